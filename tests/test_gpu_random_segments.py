@@ -1,0 +1,39 @@
+"""Sweep kernels on random segments, value for value against the oracle: every window size, windows whose
+qubits fall into one to many runs (each staging form), every matrix kind, targets and controls in every slot."""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+from qsv_b200 import engine
+from oracle import oracle as orc
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+from random_segments import random_segment, random_state  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+# (n, k, passes, ops): one tile of each size; one to a few tiles; many tiles with scattered high qubits
+SHAPES = [(10, 10, 3, 20), (11, 11, 3, 20), (12, 12, 3, 20), (13, 12, 4, 16), (14, 8, 6, 12), (17, 9, 12, 6),
+          (19, 12, 12, 8), (20, 7, 16, 4), (21, 12, 10, 10)]
+
+
+@pytest.mark.parametrize("dtype", ["c128"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_random_segments_exact(shape, dtype):
+    torch = pytest.importorskip("torch")
+    n, k, passes, ops = shape
+    old = engine.set_jit("off")
+    try:
+        for seed in range(4):
+            seg = random_segment(n, k, passes, ops, 100 * n + seed, dtype)
+            x = random_state(n, seed, dtype)
+            t = torch.from_numpy(x.copy()).cuda()
+            engine.run_segment(t, seg)
+            torch.cuda.synchronize()
+            assert engine.device_status() == 0
+            ref = orc.run_segment(x.copy(), seg)
+            assert np.array_equal(t.cpu().numpy(), ref), f"n={n} k={k} seed={seed}"
+    finally:
+        engine.set_jit(old)

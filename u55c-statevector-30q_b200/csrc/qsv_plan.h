@@ -127,8 +127,8 @@ struct QsvOpD {
 };
 
 
-// A phase's thread layout: lane bits 0-2 sit on tile bits lane_lo[0..2] (1, 2, 3 for complex64 unless the
-// sweep is swizzled, see QsvSweepT::swz; 0, 1, 2 for complex128), lane bits 3-4 on lane_bits[0..1].
+// A phase's thread layout: lane bits 0-2 sit on tile bits lane_lo[0..2] (1, 2, 3 for complex64 and 0, 1, 2
+// for complex128 unless the sweep is swizzled, see QsvSweepT::swz), lane bits 3-4 on lane_bits[0..1].
 struct QsvPhase {
     uint8_t reg_bits[QSV_RB_MAX];
     uint8_t lane_bits[2];
@@ -170,10 +170,12 @@ struct QsvSweepT {
     uint8_t H[QSV_KW_MAX];      // high window qubits, ascending
     uint8_t tma_rank;           // 0: bulk copies per sub-block; 2..5: one tensor-map box per tile
     uint8_t tdim_free[QSV_TMA_MAX_RANK];   // free bits of T folded into each tensor dim (low dim first)
-    uint8_t tdim_box[QSV_TMA_MAX_RANK];    // log2 box extent of each tensor dim
+    uint8_t tdim_box[QSV_TMA_MAX_RANK];    // log2 box extent of each tensor dim, in 8-byte elements (a
+                                           // complex128 amplitude is two: its first dim has one bit more)
     // 1: the tile sits in shared memory with the 128-byte swizzle of the tensor-map copies (16-byte chunk
-    // index = tile bits 1-3 XOR tile bits 4-6), so lane bit l may sit on tile bit 1+l or 4+l without bank
-    // conflicts and ops on tile bits 1-3 can run in registers (complex64 tensor-map sweeps only)
+    // index = tile bits 1-3 XOR tile bits 4-6; complex128: 0-2 XOR 3-5), so lane bit l may sit on tile bit
+    // 1+l or 4+l (complex128: l or 3+l) without bank conflicts and ops on tile bits 1-3 (0-2) can run in
+    // registers (tensor-map sweeps only)
     uint8_t swz;
     uint8_t pad[3];
     int64_t ntiles;             // 2^(n - kw)

@@ -103,7 +103,7 @@ int set_phase_lanes(int k) {
     return 0;
 }
 
-// swizzled layouts for complex64 tensor-map sweeps (QsvSweepT::swz): on unless QSV_SWIZZLE=0
+// swizzled layouts for tensor-map sweeps (QsvSweepT::swz): on unless QSV_SWIZZLE=0
 static bool swizzle_enabled() {
     static const bool on = [] {
         const char *e = std::getenv("QSV_SWIZZLE");
@@ -170,24 +170,29 @@ static void set_mats(QsvOpD &o, const PhysOp &p) {
 
 // Tensor-map staging for windows with short contiguous runs: one dim per chunk (<= 8 bits) of each run of
 // window bits, each spanning the free bits up to the next window bit. Returns the rank, 0 if it does not fit.
-// swz: the map of a swizzled sweep, whose first dim is exactly tile bits 0-3 (128-byte rows, the span of
-// the 128-byte swizzle); needs lo >= 4, any lo.
+// Elements are 8 bytes (the widest a tensor map has): a complex64 amplitude, or half of a complex128 one, whose
+// first dim therefore counts one bit more (half = 1) and holds at most 7 window bits.
+// swz: the map of a swizzled sweep, whose first dim is exactly 128-byte rows (the span of the 128-byte
+// swizzle): tile bits 0-3 of complex64, 0-2 of complex128; needs lo to cover them.
 template <class SW>
 static int tma_dims(const SW &sw, uint8_t *tfree, uint8_t *tbox, uint8_t *tstart, bool swz = false) {
-    if (swz ? sw.lo < 4 : sw.lo >= QSV_TMA_TENSOR_LO) return 0;
+    constexpr int half = std::is_same<typename SW::op_type, QsvOpD>::value ? 1 : 0;
+    const int row = 4 - half;              // window bits of a 128-byte row
+    if (swz ? sw.lo < row : sw.lo >= QSV_TMA_TENSOR_LO) return 0;
     int wb[QSV_KW_MAX], nw = 0;            // window bits ascending
     for (int q = 0; q < sw.lo; q++) wb[nw++] = q;
     for (int i = 0; i < sw.nh; i++) wb[nw++] = sw.H[i];
     int rank = 0, i = 0;
     while (i < nw) {
-        const int maxlen = (swz && rank == 0) ? 4 : 8;
+        const int h = rank == 0 ? half : 0;
+        const int maxlen = (swz && rank == 0) ? row : 8 - h;
         int start = wb[i], len = 1;
         while (i + len < nw && wb[i + len] == start + len && len < maxlen) len++;
         const int next = (i + len < nw) ? wb[i + len] : sw.n;
         const int fr = next - (start + len);
-        if (rank == QSV_TMA_MAX_RANK || len + fr > 31) return 0;
+        if (rank == QSV_TMA_MAX_RANK || len + h + fr > 31) return 0;
         tstart[rank] = (uint8_t)start;
-        tbox[rank] = (uint8_t)len;
+        tbox[rank] = (uint8_t)(len + h);
         tfree[rank] = (uint8_t)fr;
         rank++;
         i += len;
@@ -243,9 +248,9 @@ static void classify_ops(const std::vector<PhysOp> &ops, size_t b, size_t e, con
 // The phases of classified ops, greedy in op order, and each op's slot and layout-dependent fields. Plain
 // layout: tile bits above the fixed lane bits (>= 4 for complex64, whose tile bit 0 is the packed half of a
 // float4 and bits 1-3 are lanes; >= 3 for complex128, bits 0-2 lanes) that are targets need a register or
-// lane slot. swz (complex64 only): the swizzled layout, in which lane bit l (0-2) sits on tile bit 1+l or
-// 4+l, chosen per phase, so tile bits 1-3 need slots like the others and can be register bits; lane_cap
-// bounds its lane-bit targets (warp-shuffle ops) per phase.
+// lane slot. swz: the swizzled layout, in which lane bit l (0-2) sits on tile bit F+l or F+3+l (F = 1 for
+// complex64, 0 for complex128), chosen per phase, so tile bits F..F+2 need slots like the others and can be
+// register bits; lane_cap bounds its lane-bit targets (warp-shuffle ops) per phase.
 template <class OpT>
 static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &phases, std::string &err,
                        bool swz, int lane_cap) {
@@ -258,11 +263,10 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
         return QSV_ERR_UNSUPPORTED;
     }
     phases.clear();
-    if (C128) swz = false;
     const size_t nops = out.size();
-    // swizzled layout: tile bits 1+l and 4+l pair up on lane bit l
-    auto pair_of = [&](int t) { return (swz && t >= 1 && t <= 6) ? (t - 1) % 3 : -1; };
-    auto partner_of = [](int t) { return t <= 3 ? t + 3 : t - 3; };
+    // swizzled layout: tile bits FIXED_LO + l and FIXED_LO + 3 + l pair up on lane bit l
+    auto pair_of = [&](int t) { return (swz && t >= FIXED_LO && t < FIXED_LO + 6) ? (t - FIXED_LO) % 3 : -1; };
+    auto partner_of = [](int t) { return t < FIXED_LO + 3 ? t + 3 : t - 3; };
     struct Assign {
         int regs[QSV_RB_MAX], nr;   // register-bit targets, most used first
         int pl[3];                  // swizzled: target on lane bit l (a pair member), -1 if none
@@ -293,7 +297,7 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
         }
         return true;
     };
-    const int need_lo = swz ? 1 : FREE_LO;      // targets from this tile bit on need a slot
+    const int need_lo = swz ? FIXED_LO : FREE_LO;      // targets from this tile bit on need a slot
     size_t i = 0;
     while (i < nops) {
         size_t j = i;
@@ -329,7 +333,7 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
             int t = FIXED_LO + l;
             if (swz) {
                 if (A.pl[l] >= 0) t = A.pl[l];
-                else t = taken[1 + l] ? 4 + l : 1 + l;
+                else t = taken[FIXED_LO + l] ? FIXED_LO + 3 + l : FIXED_LO + l;
             }
             ph.lane_lo[l] = (uint8_t)t;
             taken[t] = true;
@@ -420,7 +424,7 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
         if ((qset >> q) & 1) { sw.H[nh] = (uint8_t)q; tile_of[q] = lo + nh; nh++; }
     sw.nh = nh;
     sw.ntiles = 1ll << (n - kw);
-    if (!C128) {       // complex128 tiles are staged with bulk copies only
+    {
         uint8_t tfree[QSV_TMA_MAX_RANK], tbox[QSV_TMA_MAX_RANK], tstart[QSV_TMA_MAX_RANK];
         const int r = tma_dims(sw, tfree, tbox, tstart);
         sw.tma_rank = (uint8_t)r;
@@ -436,7 +440,7 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
     // trip moves as many bytes through the shared-memory pipe as two shuffle ops); ties keep the plain one
     int plain_lane = 0;
     for (const OpT &x : vops) plain_lane += x.slot >= QSV_SLOT_LANE0 && x.variant != QSV_V_SKIP;
-    if (!C128 && swizzle_enabled() && plain_lane > 0) {
+    if (swizzle_enabled() && plain_lane > 0) {
         uint8_t tfree[QSV_TMA_MAX_RANK], tbox[QSV_TMA_MAX_RANK], tstart[QSV_TMA_MAX_RANK];
         const int r = tma_dims(sw, tfree, tbox, tstart, true);
         // QSV_PHASE_COST overrides the weight of a phase change (tuning studies)

@@ -118,8 +118,9 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// tensor map of the state for a sweep staged with one box per tile (see qsv_plan.h)
-cudaError_t make_tmap(CUtensorMap *map, float2 *state, const QsvSweep &sw) {
+// tensor map of the state for a sweep staged with one box per tile (see qsv_plan.h); 8-byte elements
+template <class SW>
+static cudaError_t make_tmap_t(CUtensorMap *map, void *state, const SW &sw) {
     std::memset(map, 0, sizeof(*map));
     if (!sw.tma_rank) return cudaSuccess;
     auto fn = encode_fn();
@@ -135,13 +136,15 @@ cudaError_t make_tmap(CUtensorMap *map, float2 *state, const QsvSweep &sw) {
         estr[d] = 1;
         start += sw.tdim_box[d] + sw.tdim_free[d];
     }
-    // a swizzled sweep's first dim is tile bits 0-3: 16 amplitudes = 128-byte rows, the 128-byte swizzle's span
+    // a swizzled sweep's first dim is 16 elements = 128-byte rows, the 128-byte swizzle's span
     if (sw.swz && (sw.tdim_box[0] != 4 || sw.tma_rank < 2)) return cudaErrorInvalidValue;
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_INT64, sw.tma_rank, state, dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, sw.swz ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
+cudaError_t make_tmap(CUtensorMap *map, float2 *state, const QsvSweep &sw) { return make_tmap_t(map, state, sw); }
+cudaError_t make_tmap(CUtensorMap *map, double2 *state, const QsvSweepD &sw) { return make_tmap_t(map, state, sw); }
 
 template <int KW, int RB, int WB, int S, int G, bool IP>
 static cudaError_t launch_stream_t(float2 *state, const QsvSweep &sw, int nsm, cudaStream_t stream) {

@@ -2,13 +2,21 @@
 //
 // No reference counterpart (the FPGA engine is complex64 only); this is the on-GPU FP64 path of the
 // precision study (a 32-qubit complex128 state is 64 GiB). Same sweep plans, addressing and staging
-// pipeline as the complex64 engine (qsv_sweep_body.cuh, bulk-async copies only), with one 16-byte
-// amplitude per thread slot: tile bits 0-2 are lane bits 0-2, two chosen tile bits are lane bits 3-4,
-// four are register bits and the rest warp bits (windows of at most 12 qubits: 3 x 64 KiB buffers).
+// pipeline as the complex64 engine (qsv_sweep_body.cuh), with one 16-byte amplitude per thread slot: tile
+// bits 0-2 are lane bits 0-2 (with the swizzled layout any of bits 0-5 can be register bits), two chosen
+// tile bits are lane bits 3-4, four are register bits and the rest warp bits (windows of at most 12 qubits:
+// 3 x 64 KiB buffers).
+// What bounds it: staging first. A window of short runs staged with one bulk copy per run (256 copies of
+// 256 bytes per 64 KiB tile each way) moved 0.9 TB/s whatever its ops; with one tensor-map box per tile the
+// same sweeps are bound by their ops. Those run in one tight loop per op variant and slot over all of a
+// thread's pairs, coefficients in registers (a class test per pair cost as much as the arithmetic).
+// A 27-qubit random-layer circuit with Toffolis, depth 8 (41 sweeps, HBM floor 27 ms): 189 ms before, 107 ms
+// with the loops, 53 ms with the tensor maps and swizzled layouts as well.
 // Every pair update is the canonical fused-multiply-add chain in double precision
 //   y0.re = fma(m00.re, x0.re, fma(-m00.im, x0.im, fma(m01.re, x1.re, -(m01.im * x1.im))))  (etc.)
 // which the CPU oracle's complex128 engine writes identically, so results agree value for value; the
 // diagonal / swap / identity forms skip exact-zero terms only.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "qsv_device.cuh"
@@ -23,112 +31,209 @@ __device__ __forceinline__ void lin_own_d(double &yr, double &yi, double ar, dou
     yr = fma(ar, owr, fma(-ai, owi, fma(br, otr, -__dmul_rn(bi, oti))));
     yi = fma(ar, owi, fma(ai, owr, fma(br, oti, __dmul_rn(bi, otr))));
 }
-__device__ __forceinline__ void diag_own_d(double &yr, double &yi, double ar, double ai, double owr, double owi) {
-    yr = fma(ar, owr, -__dmul_rn(ai, owi));
-    yi = fma(ar, owi, __dmul_rn(ai, owr));
-}
 
-// pair (x0, x1) held by one thread, matrix m of class cls
-__device__ __forceinline__ void pair_apply_d(double2 &x0, double2 &x1, const double *m, int cls) {
-    if (cls == QSV_M_DENSE) {
-        double2 y0, y1;
-        lin_own_d(y0.x, y0.y, m[0], m[1], m[2], m[3], x0.x, x0.y, x1.x, x1.y);
-        lin_own_d(y1.x, y1.y, m[6], m[7], m[4], m[5], x1.x, x1.y, x0.x, x0.y);
-        x0 = y0;
-        x1 = y1;
-    } else if (cls == QSV_M_DIAG) {
-        double2 y0, y1;
-        diag_own_d(y0.x, y0.y, m[0], m[1], x0.x, x0.y);
-        diag_own_d(y1.x, y1.y, m[6], m[7], x1.x, x1.y);
-        x0 = y0;
-        x1 = y1;
-    } else if (cls == QSV_M_DIAG1) {
-        double2 y1;
-        diag_own_d(y1.x, y1.y, m[6], m[7], x1.x, x1.y);
-        x1 = y1;
-    } else if (cls == QSV_M_XSWAP) {
-        const double2 t = x0;
-        x0 = x1;
-        x1 = t;
-    }
+// ---------------------------------------------------------------- ops by target slot
+// One uniform dispatch per op selects a tight loop over the thread's pairs, coefficients in registers. Each
+// loop computes the partial sums of all four outputs of a pair first and the final multiply-adds last, so
+// that every final is the last use of the input it replaces and can be written over its registers.
+struct MatD {
+    double m[8];
+};
+__device__ __forceinline__ void dense_d(double2 &x0, double2 &x1, const MatD &M) {
+    const double *m = M.m;
+    const double p0r = fma(-m[1], x0.y, fma(m[2], x1.x, -__dmul_rn(m[3], x1.y)));
+    const double p0i = fma(m[1], x0.x, fma(m[2], x1.y, __dmul_rn(m[3], x1.x)));
+    const double p1r = fma(-m[7], x1.y, fma(m[4], x0.x, -__dmul_rn(m[5], x0.y)));
+    const double p1i = fma(m[7], x1.x, fma(m[4], x0.y, __dmul_rn(m[5], x0.x)));
+    x0.x = fma(m[0], x0.x, p0r);
+    x0.y = fma(m[0], x0.y, p0i);
+    x1.x = fma(m[6], x1.x, p1r);
+    x1.y = fma(m[6], x1.y, p1i);
 }
-
-// own amplitude with its partner oth from the other lane; mine = 1 on the bit-1 side
-__device__ __forceinline__ void own_apply_d(double2 &own, const double2 oth, const double *m, int cls, bool mine) {
-    if (cls == QSV_M_DENSE) {
-        double2 y;
-        lin_own_d(y.x, y.y, mine ? m[6] : m[0], mine ? m[7] : m[1], mine ? m[4] : m[2], mine ? m[5] : m[3], own.x,
-                  own.y, oth.x, oth.y);
-        own = y;
-    } else if (cls == QSV_M_DIAG || (cls == QSV_M_DIAG1 && mine)) {
-        double2 y;
-        diag_own_d(y.x, y.y, mine ? m[6] : m[0], mine ? m[7] : m[1], own.x, own.y);
-        own = y;
-    } else if (cls == QSV_M_XSWAP) {
-        own = oth;
-    }
+// dense with m00 real (every U3): its two m00.im terms are exact zeros and are skipped
+__device__ __forceinline__ void dense_r0_d(double2 &x0, double2 &x1, const MatD &M) {
+    const double *m = M.m;
+    const double p0r = fma(m[2], x1.x, -__dmul_rn(m[3], x1.y));
+    const double p0i = fma(m[2], x1.y, __dmul_rn(m[3], x1.x));
+    const double p1r = fma(-m[7], x1.y, fma(m[4], x0.x, -__dmul_rn(m[5], x0.y)));
+    const double p1i = fma(m[7], x1.x, fma(m[4], x0.y, __dmul_rn(m[5], x0.x)));
+    x0.x = fma(m[0], x0.x, p0r);
+    x0.y = fma(m[0], x0.y, p0i);
+    x1.x = fma(m[6], x1.x, p1r);
+    x1.y = fma(m[6], x1.y, p1i);
 }
-
-template <int NV, int RBIT>
-__device__ __forceinline__ void reg_op_d(double2 (&A)[NV], const QsvOpD &op, const double *m0, const double *m1,
-                                         bool tok) {
-    constexpr int B = 1 << RBIT;
-    const int cm_reg = op.cm_reg, kind = op.kind, cls0 = op.cls0, cls1 = op.cls1;
+__device__ __forceinline__ void cmul_d(double2 &x, double ar, double ai) {
+    const double p = -__dmul_rn(ai, x.y), q = __dmul_rn(ai, x.x);
+    x.x = fma(ar, x.x, p);
+    x.y = fma(ar, x.y, q);
+}
+__device__ __forceinline__ MatD load_mat(const double *m) {
+    MatD M;
 #pragma unroll
-    for (int r = 0; r < NV; r++) {
-        if (r & B) continue;
-        if (kind == QSV_K_UNI) {
-            pair_apply_d(A[r], A[r | B], m0, cls0);
-            continue;
-        }
-        const bool s = tok && (r & cm_reg) == cm_reg;
-        if (s) pair_apply_d(A[r], A[r | B], m1, cls1);
-        else if (kind == QSV_K_MUX) pair_apply_d(A[r], A[r | B], m0, cls0);
-    }
+    for (int e = 0; e < 8; e++) M.m[e] = m[e];
+    return M;
 }
 
+// Register-bit target RBIT: pairs (r, r | 2^RBIT). tok: the controls outside the register bits hold.
+template <int NV, int RBIT>
+__device__ __forceinline__ void reg_op_d(double2 (&A)[NV], const QsvOpD &op, bool tok) {
+    constexpr int B = 1 << RBIT;
+    const int cm = op.cm_reg;
+#define QSV_FOR_PAIRS for (int r = 0; r < NV; r++) if (!(r & B))
+    switch (op.variant) {
+        case QSV_V_UNI_DENSE: {
+            const MatD M = load_mat(op.m0);
+            if (op.r00) {
+#pragma unroll
+                QSV_FOR_PAIRS dense_r0_d(A[r], A[r | B], M);
+            } else {
+#pragma unroll
+                QSV_FOR_PAIRS dense_d(A[r], A[r | B], M);
+            }
+            break;
+        }
+        case QSV_V_UNI_DIAG: {
+            const double ar = op.m0[0], ai = op.m0[1], br = op.m0[6], bi = op.m0[7];
+            if (op.cls == QSV_M_DIAG) {
+#pragma unroll
+                QSV_FOR_PAIRS cmul_d(A[r], ar, ai);
+            }
+#pragma unroll
+            QSV_FOR_PAIRS cmul_d(A[r | B], br, bi);
+            break;
+        }
+        case QSV_V_UNI_SWAP:
+        case QSV_V_CTRL_SWAP:
+        case QSV_V_CTRL_SWAP_SEL:
+            // lanes of a warp whose controls do not hold sit the exchange out
+            if (tok) {
+#pragma unroll
+                QSV_FOR_PAIRS if ((r & cm) == cm) { const double2 t = A[r]; A[r] = A[r | B]; A[r | B] = t; }
+            }
+            break;
+        case QSV_V_CTRL_DIAG1:
+        case QSV_V_CTRL_DIAG1_SEL: {
+            const double br = op.m1[6], bi = op.m1[7];
+            if (tok) {
+#pragma unroll
+                QSV_FOR_PAIRS if ((r & cm) == cm) cmul_d(A[r | B], br, bi);
+            }
+            break;
+        }
+        case QSV_V_CTRL_DENSE:
+        case QSV_V_CTRL_DENSE_SEL: {
+            const MatD M = load_mat(op.m1);
+            if (tok) {
+#pragma unroll
+                QSV_FOR_PAIRS if ((r & cm) == cm) dense_d(A[r], A[r | B], M);
+            }
+            break;
+        }
+        case QSV_V_MUX: {
+            const double *m0 = op.m0, *m1 = op.m1;
+#pragma unroll
+            QSV_FOR_PAIRS {
+                const bool s = tok && (r & cm) == cm;
+                MatD M;
+#pragma unroll
+                for (int e = 0; e < 8; e++) M.m[e] = s ? m1[e] : m0[e];
+                dense_d(A[r], A[r | B], M);
+            }
+            break;
+        }
+        default: break;
+    }
+#undef QSV_FOR_PAIRS
+}
+
+// Lane-bit target: each thread computes its own amplitudes as a*own + b*other, the other from the partner
+// lane, with (a, b) = (m00, m01) on the bit-0 side and (m11, m10) on the bit-1 side. Controls on register
+// bits are uniform (pairs outside them are left alone, no exchange); for controls elsewhere every lane
+// takes part in the exchange and keeps its amplitude where they do not hold.
 template <int NV>
-__device__ __forceinline__ void lane_op_d(double2 (&A)[NV], const QsvOpD &op, const double *m0, const double *m1,
-                                          bool tok, int lanebit, int lane) {
+__device__ __forceinline__ void lane_op_d(double2 (&A)[NV], const QsvOpD &op, bool tok, int lanebit, int lane) {
     const int xm = 1 << lanebit;
     const bool mine = (lane >> lanebit) & 1;
-    const int cm_reg = op.cm_reg, kind = op.kind, cls0 = op.cls0, cls1 = op.cls1;
+    const int cm = op.cm_reg;
+    auto partner = [&](const double2 &x) {
+        double2 o;
+        o.x = __shfl_xor_sync(0xffffffffu, x.x, xm);
+        o.y = __shfl_xor_sync(0xffffffffu, x.y, xm);
+        return o;
+    };
+    switch (op.variant) {
+        case QSV_V_UNI_DIAG: {
+            const double ar = mine ? op.m0[6] : op.m0[0], ai = mine ? op.m0[7] : op.m0[1];
 #pragma unroll
-    for (int r = 0; r < NV; r++) {
-        double2 oth;
-        oth.x = __shfl_xor_sync(0xffffffffu, A[r].x, xm);
-        oth.y = __shfl_xor_sync(0xffffffffu, A[r].y, xm);
-        const bool use1 = kind != QSV_K_UNI && tok && (r & cm_reg) == cm_reg;
-        if (kind == QSV_K_CTRL && !use1) continue;
-        // separate calls: a pointer select between the coefficient arrays would put them in local memory
-        if (use1) own_apply_d(A[r], oth, m1, cls1, mine);
-        else own_apply_d(A[r], oth, m0, cls0, mine);
+            for (int r = 0; r < NV; r++) cmul_d(A[r], ar, ai);
+            break;
+        }
+        case QSV_V_CTRL_DIAG1:
+        case QSV_V_CTRL_DIAG1_SEL: {
+            const double ar = op.m1[6], ai = op.m1[7];
+            if (tok && mine) {
+#pragma unroll
+                for (int r = 0; r < NV; r++)
+                    if ((r & cm) == cm) cmul_d(A[r], ar, ai);
+            }
+            break;
+        }
+        case QSV_V_UNI_SWAP:
+        case QSV_V_CTRL_SWAP:
+        case QSV_V_CTRL_SWAP_SEL:
+#pragma unroll
+            for (int r = 0; r < NV; r++)
+                if ((r & cm) == cm) {
+                    const double2 o = partner(A[r]);
+                    if (tok) A[r] = o;
+                }
+            break;
+        case QSV_V_UNI_DENSE:
+        case QSV_V_CTRL_DENSE:
+        case QSV_V_CTRL_DENSE_SEL: {
+            const double *m = op.kind == QSV_K_UNI ? op.m0 : op.m1;
+            const double ar = m[mine ? 6 : 0], ai = m[mine ? 7 : 1], br = m[mine ? 4 : 2], bi = m[mine ? 5 : 3];
+#pragma unroll
+            for (int r = 0; r < NV; r++)
+                if ((r & cm) == cm) {
+                    const double2 o = partner(A[r]);
+                    double2 y;
+                    lin_own_d(y.x, y.y, ar, ai, br, bi, A[r].x, A[r].y, o.x, o.y);
+                    if (tok) A[r] = y;
+                }
+            break;
+        }
+        case QSV_V_MUX: {
+#pragma unroll
+            for (int r = 0; r < NV; r++) {
+                const double *m = tok && (r & cm) == cm ? op.m1 : op.m0;
+                const double2 o = partner(A[r]);
+                double2 y;
+                lin_own_d(y.x, y.y, m[mine ? 6 : 0], m[mine ? 7 : 1], m[mine ? 4 : 2], m[mine ? 5 : 3], A[r].x, A[r].y,
+                          o.x, o.y);
+                A[r] = y;
+            }
+            break;
+        }
+        default: break;
     }
 }
 
 template <int NV, int RB>
 __device__ __forceinline__ void apply_op_d(const QsvOpD &op, double2 (&A)[NV], uint32_t tb, int lane) {
-    if (op.variant == QSV_V_SKIP) return;
-    double m0[8], m1[8];
-#pragma unroll
-    for (int e = 0; e < 8; e++) { m0[e] = op.m0[e]; m1[e] = op.m1[e]; }
     const bool tok = (tb & op.cm_thr) == op.cm_thr;
     const int slot = op.slot;
-    if (slot >= QSV_SLOT_LANE0) {
-        lane_op_d<NV>(A, op, m0, m1, tok, slot - QSV_SLOT_LANE0, lane);
-        return;
-    }
     switch (slot) {
-        case QSV_SLOT_REG0 + 0: reg_op_d<NV, 0>(A, op, m0, m1, tok); break;
-        case QSV_SLOT_REG0 + 1: if constexpr (RB > 1) reg_op_d<NV, (RB > 1 ? 1 : 0)>(A, op, m0, m1, tok); break;
-        case QSV_SLOT_REG0 + 2: if constexpr (RB > 2) reg_op_d<NV, (RB > 2 ? 2 : 0)>(A, op, m0, m1, tok); break;
-        case QSV_SLOT_REG0 + 3: if constexpr (RB > 3) reg_op_d<NV, (RB > 3 ? 3 : 0)>(A, op, m0, m1, tok); break;
-        default: break;
+        case QSV_SLOT_REG0 + 0: reg_op_d<NV, 0>(A, op, tok); break;
+        case QSV_SLOT_REG0 + 1: if constexpr (RB > 1) reg_op_d<NV, (RB > 1 ? 1 : 0)>(A, op, tok); break;
+        case QSV_SLOT_REG0 + 2: if constexpr (RB > 2) reg_op_d<NV, (RB > 2 ? 2 : 0)>(A, op, tok); break;
+        case QSV_SLOT_REG0 + 3: if constexpr (RB > 3) reg_op_d<NV, (RB > 3 ? 3 : 0)>(A, op, tok); break;
+        default: lane_op_d<NV>(A, op, tok, slot - QSV_SLOT_LANE0, lane); break;
     }
 }
 
-// the complex128 interpreter body: per phase, each thread loads its 2^RB amplitudes (tile bits 0-2 from
-// lane bits 0-2), applies the phase's ops and stores them back
+// the complex128 interpreter body: per phase, each thread loads its 2^RB amplitudes, applies the phase's
+// ops and stores them back
 struct InterpBodyD {
     using Amp = double2;
     static constexpr int kHalfBits = 0;
@@ -140,18 +245,27 @@ struct InterpBodyD {
         for (int ph = 0; ph < P.nphases; ph++) {
             if (ph > 0) named_bar_sync(bar, NC);
             const QsvPhase &Q = P.phases[ph];
-            uint32_t tb = (uint32_t)(lane & 7) | ((uint32_t)((lane >> 3) & 1) << Q.lane_bits[0]) |
+            uint32_t tb = ((uint32_t)(lane & 1) << Q.lane_lo[0]) | ((uint32_t)((lane >> 1) & 1) << Q.lane_lo[1]) |
+                          ((uint32_t)((lane >> 2) & 1) << Q.lane_lo[2]) |
+                          ((uint32_t)((lane >> 3) & 1) << Q.lane_bits[0]) |
                           ((uint32_t)((lane >> 4) & 1) << Q.lane_bits[1]);
 #pragma unroll
             for (int w = 0; w < WB; w++) tb |= (uint32_t)((warp >> w) & 1) << Q.warp_bits[w];
+            // slot r at tile index tb | bits of r, a swizzled tile holding amplitude x at x ^ ((x >> 3) & 7)
+            // (16-byte chunks, rows of 8): linear over XOR, so base and register offsets swizzle separately
+            const uint32_t sw = P.swz ? 7u : 0u;
+            const uint32_t base = tb ^ ((tb >> 3) & sw);
             uint32_t rbit[RB];
 #pragma unroll
-            for (int q = 0; q < RB; q++) rbit[q] = 1u << Q.reg_bits[q];
+            for (int q = 0; q < RB; q++) {
+                const uint32_t x = 1u << Q.reg_bits[q];
+                rbit[q] = x ^ ((x >> 3) & sw);
+            }
             auto pos = [&](int r) -> uint32_t {
-                uint32_t o = tb;
+                uint32_t o = base;
 #pragma unroll
                 for (int q = 0; q < RB; q++)
-                    if ((r >> q) & 1) o |= rbit[q];
+                    if ((r >> q) & 1) o ^= rbit[q];
                 return o;
             };
             double2 A[NV];
@@ -166,9 +280,12 @@ struct InterpBodyD {
 
 template <int KW, int RB, int WB, int S>
 __global__ void __launch_bounds__((1 << (5 + WB)) + 32, 1)
-    sweep_kernel_c128(double2 *__restrict__ state, const __grid_constant__ QsvSweepD P, int *status) {
-    sweep_pipeline<KW, RB, WB, S, 1, InterpBodyD, QsvSweepD>(state, P, nullptr, status);
+    sweep_kernel_c128(double2 *__restrict__ state, const __grid_constant__ QsvSweepD P,
+                      const __grid_constant__ CUtensorMap tmap, int *status) {
+    sweep_pipeline<KW, RB, WB, S, 1, InterpBodyD, QsvSweepD>(state, P, &tmap, status);
 }
+
+cudaError_t make_tmap(CUtensorMap *map, double2 *state, const QsvSweepD &sw);
 
 template <int KW, int RB, int WB, int S>
 static cudaError_t launch_c128_t(double2 *state, const QsvSweepD &sw, int nsm, int *status, cudaStream_t stream) {
@@ -188,9 +305,12 @@ static cudaError_t launch_c128_t(double2 *state, const QsvSweepD &sw, int nsm, i
         if (per_sm < 1) per_sm = 1;
         configured_dev = dev;
     }
+    alignas(64) CUtensorMap map;
+    e = make_tmap(&map, state, sw);
+    if (e != cudaSuccess) return e;
     int64_t grid = (int64_t)nsm * per_sm;
     if (grid > sw.ntiles) grid = sw.ntiles;
-    sweep_kernel_c128<KW, RB, WB, S><<<(unsigned)grid, NT, smem, stream>>>(state, sw, status);
+    sweep_kernel_c128<KW, RB, WB, S><<<(unsigned)grid, NT, smem, stream>>>(state, sw, map, status);
     return cudaGetLastError();
 }
 
@@ -199,7 +319,6 @@ static cudaError_t launch_c128_t(double2 *state, const QsvSweepD &sw, int nsm, i
 cudaError_t status_word_ptr(int **out);
 
 cudaError_t launch_sweep_c128(double2 *state, const QsvSweepD &sw, int nsm, cudaStream_t stream) {
-    if (sw.tma_rank != 0) return cudaErrorInvalidValue;        // complex128 plans stage with bulk copies
     int *status = nullptr;
     cudaError_t e = status_word_ptr(&status);
     if (e != cudaSuccess) return e;
