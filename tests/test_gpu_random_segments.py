@@ -19,7 +19,7 @@ SHAPES = [(10, 10, 3, 20), (11, 11, 3, 20), (12, 12, 3, 20), (13, 12, 4, 16), (1
           (19, 12, 12, 8), (20, 7, 16, 4), (21, 12, 10, 10)]
 
 
-@pytest.mark.parametrize("dtype", ["c128"])
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_random_segments_exact(shape, dtype):
     torch = pytest.importorskip("torch")

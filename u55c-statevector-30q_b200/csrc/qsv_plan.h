@@ -11,10 +11,11 @@
 // base | pdep(s, H)); tile T's base is pdep(T, free bits), the free bits being the qubits outside W.
 //
 // Tile staging: with long sub-blocks (lo >= QSV_TMA_TENSOR_LO) one bulk-async copy per sub-block; with
-// short ones a single tensor-map TMA box per tile. The tensor map views the state as up to 5 dims, one per
-// run of consecutive window bits (the low run [0, lo) and each run of H); every dim also spans the free
-// bits directly above its run, so a tile's free bits become box coordinates: coordinate of dim d =
-// (next tdim_free[d] bits of T) << tdim_box[d].
+// short ones tensor-map TMA boxes, one per tile when the window has few runs. The tensor map views the state
+// as up to 5 dims, one per run of consecutive window bits (the low run [0, lo) and each run of H); every dim
+// also spans the state bits directly above its run, so the address bits of a tile are its box coordinates
+// (dim d: the next tdim_box[d] + tdim_free[d] bits). When the window has more runs than dims, the last dim
+// spans all higher state bits and the tma_xbits window bits left over select one of 2^tma_xbits boxes.
 //
 // In-tile execution: consumer thread layout per phase (KW = 1 + 3 + 2 + RB + WB tile bits):
 //   tile bit 0          -> the two halves of one float4 (a thread keeps them packed as re/im float2 pairs)
@@ -168,8 +169,8 @@ struct QsvSweepT {
     int32_t lo;                 // contiguous low bits of the window
     int32_t nh;                 // |H|
     uint8_t H[QSV_KW_MAX];      // high window qubits, ascending
-    uint8_t tma_rank;           // 0: bulk copies per sub-block; 2..5: one tensor-map box per tile
-    uint8_t tdim_free[QSV_TMA_MAX_RANK];   // free bits of T folded into each tensor dim (low dim first)
+    uint8_t tma_rank;           // 0: bulk copies per sub-block; 2..5: tensor-map boxes
+    uint8_t tdim_free[QSV_TMA_MAX_RANK];   // state bits above each dim's run folded into it (low dim first)
     uint8_t tdim_box[QSV_TMA_MAX_RANK];    // log2 box extent of each tensor dim, in 8-byte elements (a
                                            // complex128 amplitude is two: its first dim has one bit more)
     // 1: the tile sits in shared memory with the 128-byte swizzle of the tensor-map copies (16-byte chunk
@@ -177,7 +178,8 @@ struct QsvSweepT {
     // 1+l or 4+l (complex128: l or 3+l) without bank conflicts and ops on tile bits 1-3 (0-2) can run in
     // registers (tensor-map sweeps only)
     uint8_t swz;
-    uint8_t pad[3];
+    uint8_t tma_xbits;          // the highest tma_xbits window bits enumerate the boxes of a tile
+    uint8_t pad[2];
     int64_t ntiles;             // 2^(n - kw)
     int32_t nphases;
     int32_t nops;

@@ -169,13 +169,22 @@ static void set_mats(QsvOpD &o, const PhysOp &p) {
 }
 
 // Tensor-map staging for windows with short contiguous runs: one dim per chunk (<= 8 bits) of each run of
-// window bits, each spanning the free bits up to the next window bit. Returns the rank, 0 if it does not fit.
+// window bits, each spanning the state bits up to the next window bit. With more chunks than dims the last
+// dim spans every higher state bit and the window bits after it (xbits of them, at most 5: boxes of at
+// least 1/32 tile, and at least the 1 KiB a swizzle pattern spans) select one of 2^xbits boxes. Returns the
+// rank, 0 if it does not fit. A bulk copy per run costs about 37 ns of the SM's copy engine whatever its
+// size, so 2^9 copies of 128 bytes per tile each way (lo = 4) ran a sweep at 1/13 of the HBM rate.
 // Elements are 8 bytes (the widest a tensor map has): a complex64 amplitude, or half of a complex128 one, whose
 // first dim therefore counts one bit more (half = 1) and holds at most 7 window bits.
 // swz: the map of a swizzled sweep, whose first dim is exactly 128-byte rows (the span of the 128-byte
 // swizzle): tile bits 0-3 of complex64, 0-2 of complex128; needs lo to cover them.
+struct TmaDims {
+    int rank = 0, xbits = 0;
+    uint8_t free[QSV_TMA_MAX_RANK], box[QSV_TMA_MAX_RANK];
+};
 template <class SW>
-static int tma_dims(const SW &sw, uint8_t *tfree, uint8_t *tbox, uint8_t *tstart, bool swz = false) {
+static int tma_dims(const SW &sw, TmaDims &D, bool swz = false) {
+    D = TmaDims();
     constexpr int half = std::is_same<typename SW::op_type, QsvOpD>::value ? 1 : 0;
     const int row = 4 - half;              // window bits of a 128-byte row
     if (swz ? sw.lo < row : sw.lo >= QSV_TMA_TENSOR_LO) return 0;
@@ -188,15 +197,19 @@ static int tma_dims(const SW &sw, uint8_t *tfree, uint8_t *tbox, uint8_t *tstart
         const int maxlen = (swz && rank == 0) ? row : 8 - h;
         int start = wb[i], len = 1;
         while (i + len < nw && wb[i + len] == start + len && len < maxlen) len++;
-        const int next = (i + len < nw) ? wb[i + len] : sw.n;
+        const bool last = rank == QSV_TMA_MAX_RANK - 1;
+        const int next = (i + len < nw && !last) ? wb[i + len] : sw.n;
         const int fr = next - (start + len);
-        if (rank == QSV_TMA_MAX_RANK || len + h + fr > 31) return 0;
-        tstart[rank] = (uint8_t)start;
-        tbox[rank] = (uint8_t)(len + h);
-        tfree[rank] = (uint8_t)fr;
+        if (len + h + fr > 31) return 0;
+        D.box[rank] = (uint8_t)(len + h);
+        D.free[rank] = (uint8_t)fr;
         rank++;
         i += len;
+        if (last) break;
     }
+    D.xbits = nw - i;
+    if (D.xbits > 5 || D.xbits > sw.nh || (D.xbits && sw.kw + half - D.xbits < 7)) return 0;
+    D.rank = rank;
     return rank;
 }
 
@@ -424,12 +437,13 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
         if ((qset >> q) & 1) { sw.H[nh] = (uint8_t)q; tile_of[q] = lo + nh; nh++; }
     sw.nh = nh;
     sw.ntiles = 1ll << (n - kw);
-    {
-        uint8_t tfree[QSV_TMA_MAX_RANK], tbox[QSV_TMA_MAX_RANK], tstart[QSV_TMA_MAX_RANK];
-        const int r = tma_dims(sw, tfree, tbox, tstart);
-        sw.tma_rank = (uint8_t)r;
-        for (int d = 0; d < r; d++) { sw.tdim_free[d] = tfree[d]; sw.tdim_box[d] = tbox[d]; }
-    }
+    auto set_dims = [&](const TmaDims &D) {
+        sw.tma_rank = (uint8_t)D.rank;
+        sw.tma_xbits = (uint8_t)D.xbits;
+        for (int d = 0; d < D.rank; d++) { sw.tdim_free[d] = D.free[d]; sw.tdim_box[d] = D.box[d]; }
+    };
+    TmaDims dims;
+    if (tma_dims(sw, dims)) set_dims(dims);
     std::vector<OpT> base, vops;
     std::vector<QsvPhaseX> vph;
     classify_ops<OpT>(ops, b, e, tile_of, n, base);
@@ -441,8 +455,7 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
     int plain_lane = 0;
     for (const OpT &x : vops) plain_lane += x.slot >= QSV_SLOT_LANE0 && x.variant != QSV_V_SKIP;
     if (swizzle_enabled() && plain_lane > 0) {
-        uint8_t tfree[QSV_TMA_MAX_RANK], tbox[QSV_TMA_MAX_RANK], tstart[QSV_TMA_MAX_RANK];
-        const int r = tma_dims(sw, tfree, tbox, tstart, true);
+        const int r = tma_dims(sw, dims, true);
         // QSV_PHASE_COST overrides the weight of a phase change (tuning studies)
         static const int phase_cost = [] {
             const char *e = std::getenv("QSV_PHASE_COST");
@@ -464,8 +477,7 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
                 vops.swap(sops);
                 vph.swap(sph);
                 sw.swz = 1;
-                sw.tma_rank = (uint8_t)r;
-                for (int d = 0; d < r; d++) { sw.tdim_free[d] = tfree[d]; sw.tdim_box[d] = tbox[d]; }
+                set_dims(dims);
             }
         }
     }

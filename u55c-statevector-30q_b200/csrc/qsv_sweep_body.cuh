@@ -2,9 +2,10 @@
 //
 // Replaces the reader / writer stages of the reference's HLS engine (kernels/sv/sv_engine.cpp:86-152,
 // DATAFLOW per pass). One persistent CTA per SM, grid-strided over the 2^(n-KW) tiles of a sweep:
-//   * a producer warp streams tiles HBM -> shared memory and back with the TMA engine: one tensor-map box
-//     per tile when the window's contiguous runs are short, one bulk-async copy per sub-block when they
-//     are long; completion is counted on mbarriers, up to S tiles are in flight;
+//   * a producer warp streams tiles HBM -> shared memory and back with the TMA engine: tensor-map boxes (one
+//     per tile, or up to 32 when the window has more runs than a tensor map has dims) when the window's
+//     contiguous runs are short, one bulk-async copy per sub-block when they are long; completion is counted
+//     on mbarriers, up to S tiles are in flight;
 //   * G groups of consumer warps run Body::tile on the staged tiles (the ops of the sweep, in registers);
 //     with G = 2 the groups take alternate tiles, so one group's phase barriers and shared-memory round
 //     trips overlap the other group's arithmetic;
@@ -135,12 +136,27 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
         const int lane = tid & 31;
         const int lo = P.lo;
         const int rank = P.tma_rank;
-        auto coords = [&](int64_t T, int32_t *c) {
-            int pos = 0;
-            for (int d = 0; d < rank; d++) {
-                const int f = P.tdim_free[d];
-                c[d] = (int32_t)(((T >> pos) & ((1ll << f) - 1)) << P.tdim_box[d]);
-                pos += f;
+        const int xbits = P.tma_xbits, nbox = 1 << xbits, boxbits = KW - xbits;
+        // coordinates of this lane's box of tile T: each dim takes the next free bits of T. With xbits > 0 the
+        // last dim also spans window bits: its free bits are spread around them, and the lane selects theirs
+        auto coords = [&](int64_t T, int32_t (&c)[QSV_TMA_MAX_RANK]) {
+            int start = 0;
+#pragma unroll
+            for (int d = 0; d < QSV_TMA_MAX_RANK; d++) {
+                if (d >= rank) break;
+                const int f = P.tdim_free[d], w = P.tdim_box[d];
+                if (d == QSV_TMA_MAX_RANK - 1 && xbits) {
+                    int64_t x = T << w;
+                    for (int i = 0; i < xbits; i++) {
+                        const int h = P.H[P.nh - xbits + i] + (int)(sizeof(Amp) / 8 - 1) - start;
+                        x = ((x >> h) << (h + 1)) | ((int64_t)((lane >> i) & 1) << h) | (x & ((1ll << h) - 1));
+                    }
+                    c[d] = (int32_t)x;
+                } else {
+                    c[d] = (int32_t)((T & ((1ll << f) - 1)) << w);
+                }
+                T >>= f;
+                start += f + w;
             }
         };
         const int nsub = 1 << (KW - lo);
@@ -162,52 +178,59 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
         };
         // fault injection (tests of the bounded waits): block 0 never loads its first tile
         const bool skip_first = P.skip_load != 0 && blockIdx.x == 0;
-        auto issue_load = [&](int64_t j, int b) {
-            const int64_t T = first + j * stride;
+        // where a tile is: its base amplitude (bulk copies) or this lane's box. Found before the wait for the
+        // tile's consumers, so that the copies go out right after it. The producer's own latency bounds the
+        // staging: with the coordinates taken from the full tile base (a loop over the window bits and arrays
+        // in local memory) every sweep took 2-3 % longer.
+        struct Place {
+            int64_t base;
+            int32_t c[QSV_TMA_MAX_RANK];
+        };
+        auto place = [&](int64_t j, Place &pl) {
+            if (rank) coords(first + j * stride, pl.c);
+            else pl.base = tile_base(first + j * stride);
+        };
+        auto issue_load = [&](int64_t j, int b, const Place &pl) {
             Amp *dst = bufs + (size_t)b * TILE;
             uint64_t *fb = &full[j % NF];
             if (skip_first && j == 0) return;
-            if (rank) {
-                if (lane == 0) {
-                    int32_t c[QSV_TMA_MAX_RANK];
-                    coords(T, c);
-                    mbar_arrive_expect_tx(fb, TILE_BYTES);
-                    tma_load(dst, tmap, c, rank, fb);
-                }
-                return;
-            }
-            const int64_t base = tile_base(T);
             if (lane == 0) mbar_arrive_expect_tx(fb, TILE_BYTES);
             __syncwarp();
-            for (int s = lane; s < nsub; s += 32) bulk_g2s(dst + (s << lo), state + (base | sub_off(s)), subbytes, fb);
+            if (rank) {                               // at most 32 boxes, one per lane
+                if (lane < nbox) tma_load(dst + (lane << boxbits), tmap, pl.c, rank, fb);
+                return;
+            }
+            for (int s = lane; s < nsub; s += 32) bulk_g2s(dst + (s << lo), state + (pl.base | sub_off(s)), subbytes, fb);
         };
-        auto issue_store = [&](int64_t j, int b) {
-            const int64_t T = first + j * stride;
+        auto issue_store = [&](int b, const Place &pl) {
             const Amp *src = bufs + (size_t)b * TILE;
             if (rank) {
-                if (lane == 0) {
-                    int32_t c[QSV_TMA_MAX_RANK];
-                    coords(T, c);
-                    tma_store(tmap, c, rank, src);
+                if (lane < nbox) {
+                    tma_store(tmap, pl.c, rank, src + (lane << boxbits));
                     bulk_commit();
                 }
                 return;
             }
-            const int64_t base = tile_base(T);
-            for (int s = lane; s < nsub; s += 32) bulk_s2g(state + (base | sub_off(s)), src + (s << lo), subbytes);
+            for (int s = lane; s < nsub; s += 32) bulk_s2g(state + (pl.base | sub_off(s)), src + (s << lo), subbytes);
             bulk_commit();
         };
+        Place ps, pl;
         int64_t issued = 0, j = 0;                    // loads issued for tiles [0, issued)
-        for (; issued < S && issued < nmine; issued++) issue_load(issued, (int)issued);
+        for (; issued < S && issued < nmine; issued++) {
+            place(issued, pl);
+            issue_load(issued, (int)issued, pl);
+        }
         for (; j < nmine; j++) {
             const int b = (int)(j % S);
             const uint32_t par = (uint32_t)((j / S) & 1);
+            place(j, ps);
+            if (j + S < nmine) place(j + S, pl);
             if (!mbar_wait(&done[b], par, &abort_flag, status, limit)) break;
-            issue_store(j, b);
+            issue_store(b, ps);
             if (j + S < nmine) {
                 bulk_wait_read_all();                 // this lane's stores have read the buffer
                 __syncwarp();
-                issue_load(j + S, b);
+                issue_load(j + S, b, pl);
                 issued = j + S + 1;
             }
         }
