@@ -16,6 +16,7 @@
 
 #include "../../include/qsv_b200.h"
 #include "qsv_device.cuh"
+#include "qsv_interp.cuh"
 #include "qsv_ops.cuh"
 #include "qsv_planner.h"
 
@@ -31,7 +32,7 @@ namespace dev {
 template <int KW, int RB, int WB, int S>
 __global__ void __launch_bounds__((1 << (5 + WB)) + 32, (KW >= 13 ? 1 : 2))
     batch_kernel(const BatchItem *__restrict__ items, int nitems, const QsvPhaseX *__restrict__ phases,
-                 const QsvOp *__restrict__ ops, int *status) {
+                 const QsvIOp *__restrict__ ops, int *status) {
     constexpr int NC = 1 << (5 + WB);
     constexpr int NV = 1 << RB;
     constexpr int TILE = 1 << KW;
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__((1 << (5 + WB)) + 32, (KW >= 13 ? 1 : 2))
 }
 
 template <int KW, int RB, int WB, int S>
-static cudaError_t launch_batch_t(const BatchItem *items, int nitems, const QsvPhaseX *phases, const QsvOp *ops,
+static cudaError_t launch_batch_t(const BatchItem *items, int nitems, const QsvPhaseX *phases, const dev::QsvIOp *ops,
                                   int *status, int nsm, cudaStream_t stream) {
     constexpr int NT = (1 << (5 + WB)) + 32;
     const size_t smem = ((size_t)S << KW) * sizeof(float2);
@@ -129,13 +130,12 @@ struct Batch {
     };
     std::vector<Circ> circs;
     std::vector<QsvPhaseX> phases;
-    std::vector<QsvOp> ops;
+    std::vector<dev::QsvIOp> ops;      // expanded for the kernel
     // finalized layout (items grouped by n, then phases, then ops, in the device workspace)
     std::vector<BatchItem> items;
     int group_off[QSV_KW_MAX + 1] = {0}, group_cnt[QSV_KW_MAX + 1] = {0};
     size_t off_phases = 0, off_ops = 0, bytes = 0;
     bool finalized = false;
-    int rb13 = 0;               // register bits of the 13-qubit layout the circuits were planned with
 };
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -149,12 +149,6 @@ int batch_add(Batch *b, void *state, int n, int nseg, const int32_t *const *segs
         if (rc) return rc;
         all.insert(all.end(), one.begin(), one.end());
     }
-    if (n == 13) {
-        int rb = 4, wb = 3;
-        layout_for_kw(13, &rb, &wb);
-        if (b->rb13 && b->rb13 != rb) { err = "13-qubit layout changed while building the batch"; return QSV_ERR_INVALID_ARG; }
-        b->rb13 = rb;
-    }
     std::vector<QsvOp> ops;
     std::vector<QsvPhaseX> phases;
     int rc = plan_whole_state(all, n, ops, phases, err);
@@ -167,7 +161,17 @@ int batch_add(Batch *b, void *state, int n, int nseg, const int32_t *const *segs
     c.ph_begin = (int32_t)b->phases.size();
     c.ph_end = c.ph_begin + (int32_t)phases.size();
     b->phases.insert(b->phases.end(), phases.begin(), phases.end());
-    b->ops.insert(b->ops.end(), ops.begin(), ops.end());
+    int rb = 0, wb = 0;
+    layout_interp(n, &rb, &wb);
+    for (const QsvOp &op : ops) {
+        dev::QsvIOp x;
+        dev::iop_header(op, 1 << rb, x);
+        for (int e = 0; e < 12; e++) {
+            x.a[e] = dev::iop_coef(op, e);
+            x.b[e] = dev::iop_coef(op, e + 12);
+        }
+        b->ops.push_back(x);
+    }
     b->circs.push_back(c);
     b->finalized = false;
     return QSV_OK;
@@ -185,7 +189,7 @@ static void batch_finalize(Batch *b) {
     }
     b->off_phases = align_up(b->items.size() * sizeof(BatchItem), 256);
     b->off_ops = align_up(b->off_phases + b->phases.size() * sizeof(QsvPhaseX), 256);
-    b->bytes = align_up(b->off_ops + b->ops.size() * sizeof(QsvOp), 256);
+    b->bytes = align_up(b->off_ops + b->ops.size() * sizeof(dev::QsvIOp), 256);
     b->finalized = true;
 }
 
@@ -204,7 +208,7 @@ cudaError_t batch_upload(Batch *b, void *ws, cudaStream_t stream) {
         e = cudaMemcpyAsync(base + b->off_phases, b->phases.data(), b->phases.size() * sizeof(QsvPhaseX),
                             cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess && !b->ops.empty())
-        e = cudaMemcpyAsync(base + b->off_ops, b->ops.data(), b->ops.size() * sizeof(QsvOp), cudaMemcpyHostToDevice,
+        e = cudaMemcpyAsync(base + b->off_ops, b->ops.data(), b->ops.size() * sizeof(dev::QsvIOp), cudaMemcpyHostToDevice,
                             stream);
     return e;
 }
@@ -214,7 +218,7 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
     char *base = static_cast<char *>(ws);
     const BatchItem *items = reinterpret_cast<const BatchItem *>(base);
     const QsvPhaseX *phases = reinterpret_cast<const QsvPhaseX *>(base + b->off_phases);
-    const QsvOp *ops = reinterpret_cast<const QsvOp *>(base + b->off_ops);
+    const dev::QsvIOp *ops = reinterpret_cast<const dev::QsvIOp *>(base + b->off_ops);
     int *status = nullptr;
     cudaError_t e = status_word_ptr(&status);
     if (e != cudaSuccess) return e;
@@ -223,14 +227,10 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
         const int cnt = b->group_cnt[n];
         if (!cnt) continue;
         const BatchItem *it = items + b->group_off[n];
-        const int rb = b->rb13 ? b->rb13 : 4;
         switch (n) {
-            case 13:
-                e = rb == 3 ? dev::launch_batch_t<13, 3, 4, 3>(it, cnt, phases, ops, status, nsm, stream)
-                            : dev::launch_batch_t<13, 4, 3, 3>(it, cnt, phases, ops, status, nsm, stream);
-                break;
-            case 12: e = dev::launch_batch_t<12, 4, 2, 3>(it, cnt, phases, ops, status, nsm, stream); break;
-            case 11: e = dev::launch_batch_t<11, 3, 2, 3>(it, cnt, phases, ops, status, nsm, stream); break;
+            case 13: e = dev::launch_batch_t<13, 3, 4, 3>(it, cnt, phases, ops, status, nsm, stream); break;
+            case 12: e = dev::launch_batch_t<12, 3, 3, 3>(it, cnt, phases, ops, status, nsm, stream); break;
+            case 11: e = dev::launch_batch_t<11, 2, 3, 3>(it, cnt, phases, ops, status, nsm, stream); break;
             default: e = dev::launch_batch_t<10, 2, 2, 3>(it, cnt, phases, ops, status, nsm, stream); break;
         }
         if (e != cudaSuccess) return e;

@@ -12,7 +12,8 @@
 #include "qsv_planner.h"
 
 namespace qsv {
-cudaError_t launch_sweep(float2 *state, const QsvSweep &sw, int nsm, cudaStream_t stream);
+cudaError_t launch_sweep(float2 *state, const QsvSweep &sw, bool planned, int nsm, cudaStream_t stream);
+bool interp_is_phase();
 int set_interp(int mode);
 cudaError_t launch_sweep_c128(double2 *state, const QsvSweepD &sw, int nsm, cudaStream_t stream);
 cudaError_t launch_remap(const void *src, void *dst, int n, const int32_t *perm, int dtype, int nsm,
@@ -35,11 +36,13 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
 cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *out, cudaStream_t stream, size_t *need);
 size_t noalloc_reduce_capacity();
 int jit_set_mode(int mode);
+int jit_mode();
 int jit_prepare(const std::vector<QsvSweep> &sweeps);
 int jit_prepare_library(const std::vector<QsvSweep> &sweeps);
 void jit_wait();
 int jit_info(long long *out, int cap);
 std::string jit_last_log();
+int jit_count_interp();
 int jit_try_launch(float2 *state, const QsvSweep &sw, int nsm, cudaStream_t stream, cudaError_t *err);
 }  // namespace qsv
 
@@ -180,17 +183,20 @@ int qsv_run_segment(void *state, int n, const int32_t *seg, size_t nwords, int d
     }
     std::vector<QsvSweep> sweeps;
     const int kw = n < QSV_KW_MAX ? n : QSV_KW_MAX;
-    rc = qsv::build_sweeps<QsvOp>(passes, n, kw, g_lo_merge, sweeps, err);
+    // with specialised kernels off the sweeps are planned for the interpreter at once
+    const bool interp = qsv::jit_mode() == 0 && qsv::interp_is_phase();
+    rc = qsv::build_sweeps<QsvOp>(passes, n, kw, g_lo_merge, sweeps, err, interp);
     if (rc) return fail(rc, err);
     std::lock_guard<std::mutex> lk(g_launch_mu);
     for (QsvSweep &sw : sweeps) {
         sw.wait_us = g_wait_us.load();
         sw.skip_load = take_injection();
         cudaError_t e = cudaSuccess;
-        const int r = qsv::jit_try_launch((float2 *)state, sw, nsm, (cudaStream_t)stream, &e);
+        const int r = interp ? qsv::jit_count_interp()
+                             : qsv::jit_try_launch((float2 *)state, sw, nsm, (cudaStream_t)stream, &e);
         if (r < 0) return cuda_fail(e, "specialised sweep launch");
         if (r == 0) {
-            e = qsv::launch_sweep((float2 *)state, sw, nsm, (cudaStream_t)stream);
+            e = qsv::launch_sweep((float2 *)state, sw, interp, nsm, (cudaStream_t)stream);
             if (e != cudaSuccess) return cuda_fail(e, "sweep launch");
         }
         t_launches++;

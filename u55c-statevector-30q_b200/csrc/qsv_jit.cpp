@@ -757,6 +757,20 @@ int jit_set_mode(int mode) {
     return old;
 }
 
+int jit_mode() {
+    Jit &j = J();
+    std::lock_guard<std::mutex> lk(j.mu);
+    return j.mode;
+}
+
+// a sweep that goes to the interpreter without asking for a specialised kernel; returns 0 as jit_try_launch does
+int jit_count_interp() {
+    Jit &j = J();
+    std::lock_guard<std::mutex> lk(j.mu);
+    j.interp_launches++;
+    return 0;
+}
+
 // Compile (in parallel, blocking) every structure of the given sweeps that is not compiled yet.
 // Returns the number of those structures whose kernel is ready.
 int jit_prepare(const std::vector<QsvSweep> &sweeps) {

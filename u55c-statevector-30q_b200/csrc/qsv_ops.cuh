@@ -377,198 +377,10 @@ __device__ __forceinline__ void comp_fixed(float2 (&R)[NV], float2 (&I)[NV], con
     }
 }
 
-template <int NV>
-__device__ __forceinline__ void lane_op_fast(float2 (&R)[NV], float2 (&I)[NV], const QsvOp &op, const float *m0,
-                                             const float *m1, bool tok, int lanebit, int lane) {
-    const int xm = 1 << lanebit;
-    const bool mine = (lane >> lanebit) & 1;
-    const int cm_reg = op.cm_reg;
-    const int var = op.variant;
-    if (var == QSV_V_UNI_DENSE || var == QSV_V_CTRL_DENSE || var == QSV_V_CTRL_DENSE_SEL) {
-        const bool uni = var == QSV_V_UNI_DENSE;
-        // value selects (a pointer select between the two coefficient arrays would put them in local memory)
-        const float a_r = uni ? (mine ? m0[6] : m0[0]) : (mine ? m1[6] : m1[0]);
-        const float a_i = uni ? (mine ? m0[7] : m0[1]) : (mine ? m1[7] : m1[1]);
-        const float b_r = uni ? (mine ? m0[4] : m0[2]) : (mine ? m1[4] : m1[2]);
-        const float b_i = uni ? (mine ? m0[5] : m0[3]) : (mine ? m1[5] : m1[3]);
-        const float2 ar = f2(a_r), ai = f2(a_i), nai = f2(-a_i), br = f2(b_r), bi = f2(b_i), nbi = f2(-b_i);
-        if (uni) {
-#pragma unroll
-            for (int r = 0; r < NV; r++) {
-                float2 oR, oI;
-                shfl4(R[r], I[r], oR, oI, xm);
-                lane_lin(R[r], I[r], oR, oI, ar, ai, nai, br, bi, nbi);
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < NV; r++) {
-                if ((r & cm_reg) != cm_reg) continue;
-                float2 oR, oI;
-                shfl4(R[r], I[r], oR, oI, xm);
-                float2 yR = R[r], yI = I[r];
-                lane_lin(yR, yI, oR, oI, ar, ai, nai, br, bi, nbi);
-                R[r] = tok ? yR : R[r];
-                I[r] = tok ? yI : I[r];
-            }
-        }
-        return;
-    }
-    if (var == QSV_V_UNI_DIAG) {
-        const float a_r = mine ? m0[6] : m0[0], a_i = mine ? m0[7] : m0[1];
-#pragma unroll
-        for (int r = 0; r < NV; r++) cmul2(R[r], I[r], a_r, a_i);
-        return;
-    }
-    if (var == QSV_V_CTRL_DIAG1 || var == QSV_V_CTRL_DIAG1_SEL) {
-        const bool s = mine && tok;
-        const float d_r = m1[6], d_i = m1[7];
-#pragma unroll
-        for (int r = 0; r < NV; r++) {
-            if ((r & cm_reg) != cm_reg) continue;
-            float2 yR = R[r], yI = I[r];
-            cmul2(yR, yI, d_r, d_i);
-            R[r] = s ? yR : R[r];
-            I[r] = s ? yI : I[r];
-        }
-        return;
-    }
-    if (var == QSV_V_UNI_SWAP || var == QSV_V_CTRL_SWAP || var == QSV_V_CTRL_SWAP_SEL) {
-        const bool uni = var == QSV_V_UNI_SWAP;
-#pragma unroll
-        for (int r = 0; r < NV; r++) {
-            if (!uni && (r & cm_reg) != cm_reg) continue;
-            float2 oR, oI;
-            shfl4(R[r], I[r], oR, oI, xm);
-            R[r] = (uni || tok) ? oR : R[r];
-            I[r] = (uni || tok) ? oI : I[r];
-        }
-        return;
-    }
-    if (var == QSV_V_SKIP) return;
-    if (var == QSV_V_MUX && op.kind == QSV_K_CTRL && op.cm_c) {
-        // M0 = identity, tile bit 0 among the controls: only the .y halves can be selected
-        if (op.cls1 == QSV_M_XSWAP) {
-#pragma unroll
-            for (int r = 0; r < NV; r++) {
-                if ((r & cm_reg) != cm_reg) continue;
-                const float oR = __shfl_xor_sync(0xffffffffu, R[r].y, xm);
-                const float oI = __shfl_xor_sync(0xffffffffu, I[r].y, xm);
-                R[r].y = tok ? oR : R[r].y;
-                I[r].y = tok ? oI : I[r].y;
-            }
-            return;
-        }
-        if (op.cls1 == QSV_M_DIAG1) {
-            const bool s = mine && tok;
-#pragma unroll
-            for (int r = 0; r < NV; r++) {
-                if ((r & cm_reg) != cm_reg) continue;
-                float yr, yi;
-                diag_own(yr, yi, m1[6], m1[7], R[r].y, I[r].y);
-                R[r].y = s ? yr : R[r].y;
-                I[r].y = s ? yi : I[r].y;
-            }
-            return;
-        }
-        if (op.cls1 == QSV_M_DENSE || op.cls1 == QSV_M_DIAG) {
-            const float a_r = mine ? m1[6] : m1[0], a_i = mine ? m1[7] : m1[1];
-            const float b_r = mine ? m1[4] : m1[2], b_i = mine ? m1[5] : m1[3];
-#pragma unroll
-            for (int r = 0; r < NV; r++) {
-                if ((r & cm_reg) != cm_reg) continue;
-                const float oR = __shfl_xor_sync(0xffffffffu, R[r].y, xm);
-                const float oI = __shfl_xor_sync(0xffffffffu, I[r].y, xm);
-                float yr, yi;
-                lin_own(yr, yi, a_r, a_i, b_r, b_i, R[r].y, I[r].y, oR, oI);
-                R[r].y = tok ? yr : R[r].y;
-                I[r].y = tok ? yi : I[r].y;
-            }
-            return;
-        }
-    }
-    lane_op<NV>(R, I, op, m0, m1, tok, lanebit, lane);
-}
-
-template <int NV, int RB>
-__device__ __forceinline__ void apply_op(const QsvOp &op, float2 (&R)[NV], float2 (&I)[NV], uint32_t tb, int lane) {
-    if (op.variant == QSV_V_SKIP) return;
-    float m0[8], m1[8];
-#pragma unroll
-    for (int e = 0; e < 8; e++) { m0[e] = op.m0[e]; m1[e] = op.m1[e]; }
-    const uint32_t cm_thr = op.cm_thr;
-    const bool thread_ok = (tb & cm_thr) == cm_thr;
-    const int slot = op.slot;
-    if (slot >= QSV_SLOT_LANE0) {
-        lane_op_fast<NV>(R, I, op, m0, m1, thread_ok, slot - QSV_SLOT_LANE0, lane);
-        return;
-    }
-    switch (slot) {
-        case QSV_SLOT_COMP: comp_op_fast<NV>(R, I, op, m0, m1, thread_ok); break;
-        case QSV_SLOT_REG0 + 0: reg_op<NV, 0>(R, I, op, m0, m1, thread_ok); break;
-        case QSV_SLOT_REG0 + 1: if constexpr (RB > 1) reg_op<NV, (RB > 1 ? 1 : 0)>(R, I, op, m0, m1, thread_ok); break;
-        case QSV_SLOT_REG0 + 2: if constexpr (RB > 2) reg_op<NV, (RB > 2 ? 2 : 0)>(R, I, op, m0, m1, thread_ok); break;
-        case QSV_SLOT_REG0 + 3: if constexpr (RB > 3) reg_op<NV, (RB > 3 ? 3 : 0)>(R, I, op, m0, m1, thread_ok); break;
-        default: break;
-    }
-}
-
 // Shared-memory position of tile index x in a swizzled tile (the tensor map's 128-byte swizzle: the 16-byte
 // chunk index, tile bits 1-3, is XORed with tile bits 4-6). Linear over XOR, so a thread's base and a
 // register offset (disjoint bits) can be swizzled separately.
 __device__ __forceinline__ uint32_t swz128(uint32_t x) { return x ^ ((x >> 3) & 0xEu); }
-
-// One phase of a tile in shared memory: read the thread's 2^RB float4 in the phase's layout, apply ops
-// [op_begin, op_end), write them back. PH is any phase record with reg_bits / lane_lo / lane_bits /
-// warp_bits; swz: the tile is stored swizzled. split_in / split_out: the slots hold (re0, re1, im0, im1),
-// the in-tile order between two phases (no repacking into the register pairs), instead of the state's
-// interleaved order (first phase in, last phase out).
-template <int NV, int RB, int WB, class PH>
-__device__ __forceinline__ void run_phase(float2 *tile, const PH &Q, const QsvOp *ops, int op_begin, int op_end,
-                                          int lane, int warp, bool swz = false, bool split_in = false,
-                                          bool split_out = false) {
-    uint32_t tb = ((uint32_t)(lane & 1) << Q.lane_lo[0]) | ((uint32_t)((lane >> 1) & 1) << Q.lane_lo[1]) |
-                  ((uint32_t)((lane >> 2) & 1) << Q.lane_lo[2]) | ((uint32_t)((lane >> 3) & 1) << Q.lane_bits[0]) |
-                  ((uint32_t)((lane >> 4) & 1) << Q.lane_bits[1]);
-#pragma unroll
-    for (int w = 0; w < WB; w++) tb |= (uint32_t)((warp >> w) & 1) << Q.warp_bits[w];
-    uint32_t rbit[RB];
-#pragma unroll
-    for (int r = 0; r < RB; r++) rbit[r] = 1u << Q.reg_bits[r];
-    auto pos = [&](int r) -> uint32_t {
-        uint32_t o = tb;
-#pragma unroll
-        for (int q = 0; q < RB; q++)
-            if ((r >> q) & 1) o |= rbit[q];
-        return o;
-    };
-    auto addr = [&](int r) -> uint32_t { return swz ? swz128(pos(r)) : pos(r); };
-    float2 R[NV], I[NV];
-    if (split_in) {
-#pragma unroll
-        for (int r = 0; r < NV; r++) {
-            const float4 v = *reinterpret_cast<const float4 *>(tile + addr(r));
-            R[r] = make_float2(v.x, v.y);
-            I[r] = make_float2(v.z, v.w);
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r < NV; r++) {
-            const float4 v = *reinterpret_cast<const float4 *>(tile + addr(r));
-            R[r] = make_float2(v.x, v.z);
-            I[r] = make_float2(v.y, v.w);
-        }
-    }
-    for (int o = op_begin; o < op_end; o++) apply_op<NV, RB>(ops[o], R, I, tb, lane);
-    if (split_out) {
-#pragma unroll
-        for (int r = 0; r < NV; r++)
-            *reinterpret_cast<float4 *>(tile + addr(r)) = make_float4(R[r].x, R[r].y, I[r].x, I[r].y);
-    } else {
-#pragma unroll
-        for (int r = 0; r < NV; r++)
-            *reinterpret_cast<float4 *>(tile + addr(r)) = make_float4(R[r].x, I[r].x, R[r].y, I[r].y);
-    }
-}
 
 }  // namespace dev
 }  // namespace qsv

@@ -128,6 +128,13 @@ int layout_for_kw(int kw, int *rb, int *wb) {
     }
 }
 
+int layout_interp(int kw, int *rb, int *wb) {
+    if (kw < 10 || kw > 13) return -1;
+    *rb = kw >= 12 ? 3 : 2;
+    *wb = kw - 6 - *rb;
+    return 0;
+}
+
 int layout_for_kw_c128(int kw, int *rb, int *wb) {
     if (kw < 10 || kw > 12) return -1;
     *rb = 4;
@@ -263,15 +270,25 @@ static void classify_ops(const std::vector<PhysOp> &ops, size_t b, size_t e, con
 // float4 and bits 1-3 are lanes; >= 3 for complex128, bits 0-2 lanes) that are targets need a register or
 // lane slot. swz: the swizzled layout, in which lane bit l (0-2) sits on tile bit F+l or F+3+l (F = 1 for
 // complex64, 0 for complex128), chosen per phase, so tile bits F..F+2 need slots like the others and can be
-// register bits; lane_cap bounds its lane-bit targets (warp-shuffle ops) per phase.
+// register bits; lane_cap bounds its lane-bit targets (warp-shuffle ops) per phase. free_diag: diagonal ops, which
+// act on each amplitude alone, need no slot (a target left on a warp bit gets QSV_SLOT_BASE), and complex64 ops
+// are laid out for the interpreter (layout_interp).
+template <class OpT>
+static bool elementwise_op(const OpT &o) {
+    return o.variant == QSV_V_SKIP || o.variant == QSV_V_UNI_DIAG || o.variant == QSV_V_CTRL_DIAG1 ||
+           o.variant == QSV_V_CTRL_DIAG1_SEL ||
+           (o.variant == QSV_V_MUX && o.kind == QSV_K_CTRL && o.cls1 == QSV_M_DIAG1);
+}
 template <class OpT>
 static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &phases, std::string &err,
-                       bool swz, int lane_cap) {
+                       bool swz, int lane_cap, bool free_diag = false) {
+    // (the callers plan for the interpreter exactly when diagonal ops need no slot)
     constexpr bool C128 = std::is_same<OpT, QsvOpD>::value;
     constexpr int FIXED_LO = C128 ? 0 : 1;       // first tile bit on lane bits 0-2
     constexpr int FREE_LO = FIXED_LO + 3;        // tile bits from here on need a slot when targeted
     int rb, wb;
-    if (C128 ? layout_for_kw_c128(kw, &rb, &wb) : layout_for_kw(kw, &rb, &wb)) {
+    if (C128 ? layout_for_kw_c128(kw, &rb, &wb)
+             : free_diag ? layout_interp(kw, &rb, &wb) : layout_for_kw(kw, &rb, &wb)) {
         err = "unsupported window size";
         return QSV_ERR_UNSUPPORTED;
     }
@@ -319,7 +336,7 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
         assign(used, cnt, 0, A);
         while (j < nops) {
             const int tb = out[j].tbit;
-            if (tb >= need_lo) {
+            if (tb >= need_lo && !(free_diag && elementwise_op(out[j]))) {
                 int f = -1;
                 for (int u = 0; u < nu; u++)
                     if (used[u] == tb) f = u;
@@ -385,6 +402,7 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
                     if (ph.lane_lo[l] == tb) op.slot = (uint8_t)(QSV_SLOT_LANE0 + l);
                 for (int l = 0; l < 2; l++)
                     if (ph.lane_bits[l] == tb) op.slot = (uint8_t)(QSV_SLOT_LANE0 + 3 + l);
+                if (op.slot == 0xff && free_diag && elementwise_op(op)) op.slot = QSV_SLOT_BASE;
                 if (op.slot == 0xff) { err = "internal: target not placed"; return QSV_ERR_UNSUPPORTED; }
             }
             // control split for this phase's layout: register-index part, tile-bit-0 part, thread part
@@ -409,62 +427,45 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
 template <class OpT>
 static int plan_window(const std::vector<PhysOp> &ops, size_t b, size_t e, const int *tile_of, int n, int kw,
                        std::vector<OpT> &out, std::vector<QsvPhaseX> &phases, std::string &err, bool swz = false,
-                       int lane_cap = 8) {
+                       int lane_cap = 8, bool free_diag = false) {
     classify_ops<OpT>(ops, b, e, tile_of, n, out);
-    return plan_phases<OpT>(out, kw, phases, err, swz, lane_cap);
+    return plan_phases<OpT>(out, kw, phases, err, swz, lane_cap, free_diag);
 }
 
+// The phases of a sweep's classified ops (window and n set), in the plain layout or a swizzled one.
 template <class OpT>
-static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64_t qset, int n, int kw,
-                      QsvSweepT<OpT> &sw, std::string &err) {
-    constexpr bool C128 = std::is_same<OpT, QsvOpD>::value;
-    int rb, wb;
-    if (C128 ? layout_for_kw_c128(kw, &rb, &wb) : layout_for_kw(kw, &rb, &wb)) {
-        err = "unsupported window size";
-        return QSV_ERR_UNSUPPORTED;
-    }
-    std::memset(&sw, 0, sizeof(sw));
-    const int lo = window_lo(qset, n, kw);
-    if (lo < QSV_LO_MIN) { err = "op qubits do not fit one 13-qubit window"; return QSV_ERR_UNSUPPORTED; }
-    sw.n = n;
-    sw.kw = kw;
-    sw.lo = lo;
-    int tile_of[64];
-    for (int q = 0; q < 64; q++) tile_of[q] = -1;
-    for (int q = 0; q < lo; q++) tile_of[q] = q;
-    int nh = 0;
-    for (int q = lo; q < n; q++)
-        if ((qset >> q) & 1) { sw.H[nh] = (uint8_t)q; tile_of[q] = lo + nh; nh++; }
-    sw.nh = nh;
-    sw.ntiles = 1ll << (n - kw);
+static int choose_layout(QsvSweepT<OpT> &sw, const std::vector<OpT> &base, bool free_diag, std::string &err) {
+    const int kw = sw.kw;
     auto set_dims = [&](const TmaDims &D) {
         sw.tma_rank = (uint8_t)D.rank;
         sw.tma_xbits = (uint8_t)D.xbits;
         for (int d = 0; d < D.rank; d++) { sw.tdim_free[d] = D.free[d]; sw.tdim_box[d] = D.box[d]; }
     };
     TmaDims dims;
+    sw.swz = 0;
+    sw.tma_rank = sw.tma_xbits = 0;
     if (tma_dims(sw, dims)) set_dims(dims);
-    std::vector<OpT> base, vops;
+    std::vector<OpT> vops = base;
     std::vector<QsvPhaseX> vph;
-    classify_ops<OpT>(ops, b, e, tile_of, n, base);
-    vops = base;
-    int rc = plan_phases<OpT>(vops, kw, vph, err, false, 8);
+    int rc = plan_phases<OpT>(vops, kw, vph, err, false, 8, free_diag);
     if (rc) return rc;
+    auto lane_ops = [&](const std::vector<OpT> &o) {
+        int lane = 0;
+        for (const OpT &x : o)
+            lane += x.slot >= QSV_SLOT_LANE0 && x.variant != QSV_V_SKIP && !(free_diag && elementwise_op(x));
+        return lane;
+    };
     // the swizzled layout where it costs less: cost = lane ops + 2 per phase change (a shared-memory round
     // trip moves as many bytes through the shared-memory pipe as two shuffle ops); ties keep the plain one
-    int plain_lane = 0;
-    for (const OpT &x : vops) plain_lane += x.slot >= QSV_SLOT_LANE0 && x.variant != QSV_V_SKIP;
-    if (swizzle_enabled() && plain_lane > 0) {
+    if (swizzle_enabled() && (lane_ops(vops) > 0 || (free_diag && vph.size() > 1))) {
         const int r = tma_dims(sw, dims, true);
         // QSV_PHASE_COST overrides the weight of a phase change (tuning studies)
         static const int phase_cost = [] {
             const char *e = std::getenv("QSV_PHASE_COST");
             return e ? std::atoi(e) : 2;
         }();
-        auto cost = [](const std::vector<OpT> &o, const std::vector<QsvPhaseX> &p) {
-            int lane = 0;
-            for (const OpT &x : o) lane += x.slot >= QSV_SLOT_LANE0 && x.variant != QSV_V_SKIP;
-            return lane + phase_cost * ((int)p.size() - 1);
+        auto cost = [&](const std::vector<OpT> &o, const std::vector<QsvPhaseX> &p) {
+            return lane_ops(o) + phase_cost * ((int)p.size() - 1);
         };
         // phases with fewer shuffle ops but more round trips, or the reverse: try lane-op budgets per phase
         for (int cap : {0, 1, 2, 8}) {
@@ -472,7 +473,7 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
             std::vector<OpT> sops = base;
             std::vector<QsvPhaseX> sph;
             std::string serr;
-            if (plan_phases<OpT>(sops, kw, sph, serr, true, cap) == QSV_OK &&
+            if (plan_phases<OpT>(sops, kw, sph, serr, true, cap, free_diag) == QSV_OK &&
                 sph.size() <= QSV_MAX_PHASES && cost(sops, sph) < cost(vops, vph)) {
                 vops.swap(sops);
                 vph.swap(sph);
@@ -498,18 +499,57 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
     return QSV_OK;
 }
 
+template <class OpT>
+static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64_t qset, int n, int kw,
+                      QsvSweepT<OpT> &sw, std::string &err, bool interp) {
+    constexpr bool C128 = std::is_same<OpT, QsvOpD>::value;
+    int rb, wb;
+    if (C128 ? layout_for_kw_c128(kw, &rb, &wb) : layout_for_kw(kw, &rb, &wb)) {
+        err = "unsupported window size";
+        return QSV_ERR_UNSUPPORTED;
+    }
+    std::memset(&sw, 0, sizeof(sw));
+    const int lo = window_lo(qset, n, kw);
+    if (lo < QSV_LO_MIN) { err = "op qubits do not fit one 13-qubit window"; return QSV_ERR_UNSUPPORTED; }
+    sw.n = n;
+    sw.kw = kw;
+    sw.lo = lo;
+    int tile_of[64];
+    for (int q = 0; q < 64; q++) tile_of[q] = -1;
+    for (int q = 0; q < lo; q++) tile_of[q] = q;
+    int nh = 0;
+    for (int q = lo; q < n; q++)
+        if ((qset >> q) & 1) { sw.H[nh] = (uint8_t)q; tile_of[q] = lo + nh; nh++; }
+    sw.nh = nh;
+    sw.ntiles = 1ll << (n - kw);
+    std::vector<OpT> base;
+    classify_ops<OpT>(ops, b, e, tile_of, n, base);
+    // complex128 sweeps only ever run on their interpreter
+    return choose_layout<OpT>(sw, base, C128 || interp, err);
+}
+
+int plan_interp(QsvSweep &sw, std::string &err) {
+    std::vector<QsvOp> base(sw.ops, sw.ops + sw.nops);
+    for (QsvOp &op : base) {                   // as classified: the branch-free forms depend on the layout
+        if (op.variant == QSV_V_CTRL_DENSE_SEL) op.variant = QSV_V_CTRL_DENSE;
+        else if (op.variant == QSV_V_CTRL_DIAG1_SEL) op.variant = QSV_V_CTRL_DIAG1;
+        else if (op.variant == QSV_V_CTRL_SWAP_SEL) op.variant = QSV_V_CTRL_SWAP;
+    }
+    return choose_layout<QsvOp>(sw, base, true, err);
+}
+
 int plan_whole_state(const std::vector<PhysPass> &passes, int n, std::vector<QsvOp> &ops_out,
                      std::vector<QsvPhaseX> &phases_out, std::string &err) {
     std::vector<PhysOp> ops;
     for (const PhysPass &p : passes) ops.insert(ops.end(), p.ops.begin(), p.ops.end());
     int tile_of[64];
     for (int q = 0; q < 64; q++) tile_of[q] = q < n ? q : -1;
-    return plan_window<QsvOp>(ops, 0, ops.size(), tile_of, n, n, ops_out, phases_out, err);
+    return plan_window<QsvOp>(ops, 0, ops.size(), tile_of, n, n, ops_out, phases_out, err, false, 8, true);
 }
 
 template <class OpT>
 int build_sweeps(const std::vector<PhysPass> &passes, int n, int kw, int lo_merge,
-                 std::vector<QsvSweepT<OpT>> &out, std::string &err) {
+                 std::vector<QsvSweepT<OpT>> &out, std::string &err, bool interp) {
     out.clear();
     std::vector<PhysOp> ops;
     uint64_t cur = 0;
@@ -517,7 +557,7 @@ int build_sweeps(const std::vector<PhysPass> &passes, int n, int kw, int lo_merg
     auto flush = [&]() -> int {
         if (ops.size() > begin) {
             out.emplace_back();
-            int rc = fill_sweep<OpT>(ops, begin, ops.size(), cur, n, kw, out.back(), err);
+            int rc = fill_sweep<OpT>(ops, begin, ops.size(), cur, n, kw, out.back(), err, interp);
             if (rc) return rc;
         }
         begin = ops.size();
@@ -541,9 +581,9 @@ int build_sweeps(const std::vector<PhysPass> &passes, int n, int kw, int lo_merg
     return flush();
 }
 template int build_sweeps<QsvOp>(const std::vector<PhysPass> &, int, int, int, std::vector<QsvSweep> &,
-                                 std::string &);
+                                 std::string &, bool);
 template int build_sweeps<QsvOpD>(const std::vector<PhysPass> &, int, int, int, std::vector<QsvSweepD> &,
-                                  std::string &);
+                                  std::string &, bool);
 
 // Groups for the streaming interpreter, greedy in op order: a group takes ops while their targets (tile
 // bits >= 1, except diagonal ops, which act element by element and so run on any tile bit of the item)

@@ -35,7 +35,11 @@ int decode_segment(const int32_t *seg, size_t nwords, int n, std::vector<PhysPas
                    int dtype = 0);
 // Register/warp bit split of the consumer layout for a window of kw qubits (kw in 10..13).
 int layout_for_kw(int kw, int *rb, int *wb);
-// Choose the 13-qubit layout: 4 register bits x 8 consumer warps, or 3 x 16 (process-wide).
+// The interpreter's split (sweep and batch kernels): at most 3 register bits, so that its 16-warp (13 qubits)
+// blocks hide the latency of the per-op dispatch (8 warps with 4 register bits issued 1.5 instructions per cycle
+// and SM, 16 warps 2.2).
+int layout_interp(int kw, int *rb, int *wb);
+// Choose the 13-qubit layout of specialised kernels: 4 register bits x 8 consumer warps, or 3 x 16 (process-wide).
 int set_rb13(int rb);
 // How many of a phase's targets (tile bits >= 4) may sit on lane bits 3, 4 (0..2; default 1).
 int set_phase_lanes(int k);
@@ -44,13 +48,18 @@ int set_phase_lanes(int k);
 int layout_for_kw_c128(int kw, int *rb, int *wb);
 // Merge consecutive passes into sweeps of window kw; merged windows keep >= 2^lo_merge contiguous amps.
 // OpT = QsvOp (complex64) or QsvOpD (complex128).
+// interp: complex64 sweeps are planned for the interpreter at once (as plan_interp would).
 template <class OpT>
 int build_sweeps(const std::vector<PhysPass> &passes, int n, int kw, int lo_merge,
-                 std::vector<QsvSweepT<OpT>> &out, std::string &err);
+                 std::vector<QsvSweepT<OpT>> &out, std::string &err, bool interp = false);
 // Whole-state program of an n-qubit circuit (n in 10..13: the state is one tile): every op of every pass,
 // in order, with its phases.
 int plan_whole_state(const std::vector<PhysPass> &passes, int n, std::vector<QsvOp> &ops_out,
                      std::vector<QsvPhaseX> &phases_out, std::string &err);
+// Re-plan the phases of a complex64 sweep for the interpreter, whose diagonal ops run wherever their target sits
+// (QSV_SLOT_BASE on a warp bit): only the other ops' targets need register or lane slots. Layout:
+// layout_interp.
+int plan_interp(QsvSweep &sw, std::string &err);
 // Re-plan a complex64 sweep for the streaming interpreter: groups of consecutive ops with at most three
 // distinct target tile bits >= 1 (ops on tile bit 0 and diagonal ops on other bits join any group), and
 // each op's slot / control split for its group's item layout. Replaces the phase fields of the ops.

@@ -4,12 +4,12 @@
 // writer :120-152 DATAFLOW per pass). The staging pipeline (persistent CTA per SM, producer warp with
 // TMA / bulk-async copies, mbarrier hand-offs) is qsv_sweep_body.cuh; this file supplies the interpreter
 // body and the host launchers:
-//   * consumer warps apply the sweep's ops in registers. A thread keeps 2^RB float4 (the two halves of
-//     each float4 = tile bit 0) repacked as float2 (re, re) / (im, im) pairs so that every register-bit op
-//     runs on two amplitude pairs per packed FP32x2 FMA; ops on lane bits exchange with warp shuffles; an op
-//     whose target is on a warp bit starts a new phase (shared-memory round trip in another layout);
-//   * the interpreter reads each op's slot and variant at run time; qsv_jit.cpp compiles kernels with the
-//     same body specialised to one sweep structure and launches those when they are ready.
+//   * consumer warps apply the sweep's ops in registers (qsv_interp.cuh): a thread keeps 2^RB slots as packed
+//     (re, re) / (im, im) 64-bit registers so that every register-bit op runs on two amplitude pairs per packed
+//     FP32x2 FMA; ops on lane bits exchange with warp shuffles; an op whose target is on a warp bit starts a new
+//     phase (shared-memory round trip in another layout) unless it is diagonal;
+//   * the interpreter finds each op's code path at run time; qsv_jit.cpp compiles kernels with the
+//     same arithmetic specialised to one sweep structure and launches those when they are ready.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -20,6 +20,7 @@
 #include <string>
 
 #include "qsv_device.cuh"
+#include "qsv_interp.cuh"
 #include "qsv_ops.cuh"
 #include "qsv_planner.h"
 #include "qsv_stream.cuh"
@@ -37,14 +38,30 @@ struct InterpBody {
     using Amp = float2;
     static constexpr int kHalfBits = 1;
     static constexpr bool kSmemOps = true;
+    using IOp = QsvIOp;
+    // the expanded table follows the raw one
+    static __device__ __forceinline__ QsvIOp *table(const QsvOp *sops) {
+        return reinterpret_cast<QsvIOp *>(const_cast<QsvOp *>(sops) + QSV_MAX_SWEEP_OPS);
+    }
+    template <int NV>
+    static __device__ __forceinline__ void expand(const QsvOp *sops, int nops, int tid, int nthreads) {
+        QsvIOp *t = table(sops);
+        // one coefficient or header per thread and turn (25 pieces per op)
+        for (int i = tid; i < nops * 25; i += nthreads) {
+            const int o = i / 25, e = i - o * 25;
+            if (e == 24) iop_header(sops[o], NV, t[o]);
+            else (e < 12 ? t[o].a : t[o].b - 12)[e] = iop_coef(sops[o], e);
+        }
+    }
     template <int NV, int RB, int WB>
     static __device__ __forceinline__ void tile(float2 *tile, const QsvSweep &P, const QsvOp *sops, int lane, int warp,
                                                 int bar) {
         constexpr int NC = 1 << (5 + WB);
+        const QsvIOp *iops = table(sops);
         for (int ph = 0; ph < P.nphases; ph++) {
             if (ph > 0) named_bar_sync(bar, NC);
             const QsvPhase &Q = P.phases[ph];
-            run_phase<NV, RB, WB>(tile, Q, sops, Q.op_begin, Q.op_end, lane, warp, P.swz != 0, ph > 0,
+            run_phase<NV, RB, WB>(tile, Q, iops, Q.op_begin, Q.op_end, lane, warp, P.swz != 0, ph > 0,
                                   ph + 1 < P.nphases);
         }
     }
@@ -261,16 +278,22 @@ static cudaError_t launch_stream(float2 *state, const QsvSweep &sw, int nsm, cud
     }
 }
 
-cudaError_t launch_sweep(float2 *state, const QsvSweep &sw, int nsm, cudaStream_t stream) {
-    if (g_interp.load(std::memory_order_relaxed) == 1) return launch_stream(state, sw, nsm, stream);
-    int rb = 4, wb = 3;
-    layout_for_kw(sw.kw, &rb, &wb);
+bool interp_is_phase() { return g_interp.load(std::memory_order_relaxed) == 0; }
+
+// sw: planned for specialised kernels, or for the phase interpreter (planned)
+cudaError_t launch_sweep(float2 *state, const QsvSweep &sw_in, bool planned, int nsm, cudaStream_t stream) {
+    if (!planned && !interp_is_phase()) return launch_stream(state, sw_in, nsm, stream);
+    thread_local QsvSweep own;
+    if (!planned) {
+        std::memcpy(&own, &sw_in, offsetof(QsvSweep, ngroups));
+        std::string err;
+        if (plan_interp(own, err) != QSV_OK) return cudaErrorInvalidValue;
+    }
+    const QsvSweep &sw = planned ? sw_in : own;
     switch (sw.kw) {
-        case 13:
-            if (rb == 3) return dev::launch_sweep_t<13, 3, 4, 3>(state, sw, nsm, stream);
-            return dev::launch_sweep_t<13, 4, 3, 3>(state, sw, nsm, stream);
-        case 12: return dev::launch_sweep_t<12, 4, 2, 3>(state, sw, nsm, stream);
-        case 11: return dev::launch_sweep_t<11, 3, 2, 3>(state, sw, nsm, stream);
+        case 13: return dev::launch_sweep_t<13, 3, 4, 3>(state, sw, nsm, stream);
+        case 12: return dev::launch_sweep_t<12, 3, 3, 3>(state, sw, nsm, stream);
+        case 11: return dev::launch_sweep_t<11, 2, 3, 3>(state, sw, nsm, stream);
         case 10: return dev::launch_sweep_t<10, 2, 2, 3>(state, sw, nsm, stream);
         default: return cudaErrorInvalidValue;
     }

@@ -69,13 +69,31 @@ __device__ __forceinline__ void tma_store(const CUtensorMap *map, const int32_t 
     }
 }
 
+// A body that reads its ops in another form names that record type IOp and fills the table, which follows the
+// raw one in shared memory, with expand(): the consumers do it while the first tiles are on their way.
+template <class T>
+struct VoidOf {
+    typedef void type;
+};
+template <class Body, class = void>
+struct ExpandedOps {
+    static constexpr bool value = false;
+    static constexpr size_t bytes = 0;
+};
+template <class Body>
+struct ExpandedOps<Body, typename VoidOf<typename Body::IOp>::type> {
+    static constexpr bool value = true;
+    static constexpr size_t bytes = sizeof(typename Body::IOp) * QSV_MAX_SWEEP_OPS;
+};
+
 // Dynamic shared memory a sweep kernel needs: S tile buffers, plus the op table when Body reads it there,
 // plus 1 KiB to align the buffers to 1024 bytes (the 128-byte swizzle pattern repeats every 1024 bytes of
 // shared-memory address, and the consumers' addressing assumes it starts at each buffer).
 template <int KW, int S, class Body, class SW = QsvSweep>
 __host__ __device__ constexpr size_t sweep_smem_bytes() {
     return ((size_t)S << KW) * sizeof(typename Body::Amp) +
-           (Body::kSmemOps ? sizeof(typename SW::op_type) * QSV_MAX_SWEEP_OPS : 0) + QSV_SMEM_ALIGN;
+           (Body::kSmemOps ? sizeof(typename SW::op_type) * QSV_MAX_SWEEP_OPS : 0) + ExpandedOps<Body>::bytes +
+           QSV_SMEM_ALIGN;
 }
 
 // The pipeline. Launch with G * (1 << (5 + WB)) + 32 threads and sweep_smem_bytes<KW, S, Body, SW>() bytes
@@ -245,6 +263,10 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
     }
 
     // ---------------------------------------------------------------- consumer warps
+    if constexpr (ExpandedOps<Body>::value) {
+        Body::template expand<NV>(sops, P.nops, tid, NC);
+        named_bar_sync(1, NC);
+    }
     if constexpr (IL != 0) {
         static_assert(G == 1, "interleaved phases run one consumer group");
         // tiles j0 and j0 + 1 (slots u = 0, 1): phase p of both, then phase p + 1 of both. Every consumer

@@ -92,16 +92,6 @@ __device__ __forceinline__ void reg_op_d(double2 (&A)[NV], const QsvOpD &op, boo
             }
             break;
         }
-        case QSV_V_UNI_DIAG: {
-            const double ar = op.m0[0], ai = op.m0[1], br = op.m0[6], bi = op.m0[7];
-            if (op.cls == QSV_M_DIAG) {
-#pragma unroll
-                QSV_FOR_PAIRS cmul_d(A[r], ar, ai);
-            }
-#pragma unroll
-            QSV_FOR_PAIRS cmul_d(A[r | B], br, bi);
-            break;
-        }
         case QSV_V_UNI_SWAP:
         case QSV_V_CTRL_SWAP:
         case QSV_V_CTRL_SWAP_SEL:
@@ -111,15 +101,6 @@ __device__ __forceinline__ void reg_op_d(double2 (&A)[NV], const QsvOpD &op, boo
                 QSV_FOR_PAIRS if ((r & cm) == cm) { const double2 t = A[r]; A[r] = A[r | B]; A[r | B] = t; }
             }
             break;
-        case QSV_V_CTRL_DIAG1:
-        case QSV_V_CTRL_DIAG1_SEL: {
-            const double br = op.m1[6], bi = op.m1[7];
-            if (tok) {
-#pragma unroll
-                QSV_FOR_PAIRS if ((r & cm) == cm) cmul_d(A[r | B], br, bi);
-            }
-            break;
-        }
         case QSV_V_CTRL_DENSE:
         case QSV_V_CTRL_DENSE_SEL: {
             const MatD M = load_mat(op.m1);
@@ -162,22 +143,6 @@ __device__ __forceinline__ void lane_op_d(double2 (&A)[NV], const QsvOpD &op, bo
         return o;
     };
     switch (op.variant) {
-        case QSV_V_UNI_DIAG: {
-            const double ar = mine ? op.m0[6] : op.m0[0], ai = mine ? op.m0[7] : op.m0[1];
-#pragma unroll
-            for (int r = 0; r < NV; r++) cmul_d(A[r], ar, ai);
-            break;
-        }
-        case QSV_V_CTRL_DIAG1:
-        case QSV_V_CTRL_DIAG1_SEL: {
-            const double ar = op.m1[6], ai = op.m1[7];
-            if (tok && mine) {
-#pragma unroll
-                for (int r = 0; r < NV; r++)
-                    if ((r & cm) == cm) cmul_d(A[r], ar, ai);
-            }
-            break;
-        }
         case QSV_V_UNI_SWAP:
         case QSV_V_CTRL_SWAP:
         case QSV_V_CTRL_SWAP_SEL:
@@ -219,10 +184,77 @@ __device__ __forceinline__ void lane_op_d(double2 (&A)[NV], const QsvOpD &op, bo
     }
 }
 
+// Diagonal ops act on each amplitude alone, so their target may sit anywhere. With the target in the thread
+// (slots differ) or not (the thread's bit decides), diag(a, b) is a factor on the slots without and one on
+// the slots with it; controlled ops are diag(1, d): a factor on the slots with target and controls set.
+template <int NV, int RM>
+__device__ __forceinline__ void phase_slots_d(double2 (&A)[NV], double ar, double ai) {
+#pragma unroll
+    for (int r = 0; r < NV; r++)
+        if ((r & RM) == RM) cmul_d(A[r], ar, ai);
+}
+template <int NV, int RB>
+__device__ __forceinline__ void diag_op_d(double2 (&A)[NV], const QsvOpD &op, uint32_t tb) {
+    const int slot = op.slot;
+    const bool reg = slot < QSV_SLOT_BASE, uni = op.kind == QSV_K_UNI;
+    int rm = op.cm_reg;
+    uint32_t thr = op.cm_thr;
+    if (reg) rm |= 1 << (slot - QSV_SLOT_REG0);
+    else thr |= 1u << op.tbit;
+    const bool on = (tb & thr) == thr;
+    const double *m = uni ? op.m0 : op.m1;
+    if (uni && op.cls == QSV_M_DIAG && (reg || !on)) {       // the amplitudes with the target bit clear
+        const double ar = m[0], ai = m[1];
+        switch (reg ? rm : 0) {
+            case 0: phase_slots_d<NV, 0>(A, ar, ai); break;
+            case 1:
+#pragma unroll
+                for (int r = 0; r < NV; r++) if (!(r & 1)) cmul_d(A[r], ar, ai);
+                break;
+            case 2:
+#pragma unroll
+                for (int r = 0; r < NV; r++) if (!(r & 2)) cmul_d(A[r], ar, ai);
+                break;
+            case 4:
+#pragma unroll
+                for (int r = 0; r < NV; r++) if (!(r & 4)) cmul_d(A[r], ar, ai);
+                break;
+            default:
+#pragma unroll
+                for (int r = 0; r < NV; r++) if (!(r & 8)) cmul_d(A[r], ar, ai);
+                break;
+        }
+    }
+    if (!on) return;
+    const double br = m[6], bi = m[7];
+    switch (rm) {
+        case 0: phase_slots_d<NV, 0>(A, br, bi); break;
+        case 1: phase_slots_d<NV, 1>(A, br, bi); break;
+        case 2: phase_slots_d<NV, 2>(A, br, bi); break;
+        case 3: phase_slots_d<NV, 3>(A, br, bi); break;
+        case 4: phase_slots_d<NV, 4>(A, br, bi); break;
+        case 5: phase_slots_d<NV, 5>(A, br, bi); break;
+        case 6: phase_slots_d<NV, 6>(A, br, bi); break;
+        case 8: phase_slots_d<NV, 8>(A, br, bi); break;
+        case 9: phase_slots_d<NV, 9>(A, br, bi); break;
+        case 10: phase_slots_d<NV, 10>(A, br, bi); break;
+        case 12: phase_slots_d<NV, 12>(A, br, bi); break;
+        default:
+#pragma unroll
+            for (int r = 7; r < NV; r++)
+                if ((r & rm) == rm) cmul_d(A[r], br, bi);
+            break;
+    }
+}
+
 template <int NV, int RB>
 __device__ __forceinline__ void apply_op_d(const QsvOpD &op, double2 (&A)[NV], uint32_t tb, int lane) {
+    const int slot = op.slot, v = op.variant;
+    if (v == QSV_V_UNI_DIAG || v == QSV_V_CTRL_DIAG1 || v == QSV_V_CTRL_DIAG1_SEL) {
+        diag_op_d<NV, RB>(A, op, tb);
+        return;
+    }
     const bool tok = (tb & op.cm_thr) == op.cm_thr;
-    const int slot = op.slot;
     switch (slot) {
         case QSV_SLOT_REG0 + 0: reg_op_d<NV, 0>(A, op, tok); break;
         case QSV_SLOT_REG0 + 1: if constexpr (RB > 1) reg_op_d<NV, (RB > 1 ? 1 : 0)>(A, op, tok); break;
