@@ -157,100 +157,228 @@ __global__ void set_amp0_kernel(float2 *state) { state[0] = make_float2(1.0f, 0.
 __global__ void set_amp0_kernel_d(double2 *state) { state[0] = make_double2(1.0, 0.0); }
 
 // ---------------------------------------------------------------- FP64 reductions
-// Block b covers amplitudes [b << B, (b+1) << B). Thread t visits i = (b << B) + t + 256 * it. The
-// per-block result is 1 + B doubles: the block total and, for each bit q < B of the index, the sum of
-// |a_i|^2 over the block's i with bit q set. Fixed summation order (deterministic).
+// Sum |a|^2 and, for every index bit q, the sum over the indices with bit q set. A block takes chunks of 2^13
+// amplitudes (256 threads, 16-byte loads, 16 in flight per thread: 16 float4 of two complex64 amplitudes each,
+// or 2 x 16 double2). A chunk's index bits are: bits in the 16-byte vector (complex64), 8 thread bits, 4 (5)
+// load bits, and the chunk number above. Per-bit sums of the load bits share one addition tree; a bit of the
+// thread or the chunk number selects whole-thread sums. Fixed summation order (deterministic).
+// What bounds it: HBM. One read of the state, about 4 FP64 operations and 2 conversions per amplitude. With
+// the per-bit sums in a run-time-indexed array (local memory) a 30-qubit complex64 reduction took 2.61 ms,
+// half the HBM rate; now 1.23 ms (7.0 TB/s, reads only).
 #define RED_THREADS 256
-template <class A>
-__global__ void __launch_bounds__(RED_THREADS)
-    reduce_block_kernel(const A *__restrict__ state, int B, double *__restrict__ partials) {
-    __shared__ double s_tot[RED_THREADS];
-    __shared__ double s_bits[RED_THREADS][17];
-    const int t = threadIdx.x;
-    const int64_t base = (int64_t)blockIdx.x << B;
-    const int niter = 1 << (B - 8);
-    double tot = 0.0;
-    double hb[17];                  // bits 8..B-1 of i (from it)
+#define RED_CHUNK_BITS 13
+#define RED_HI 21                  // bits above a chunk: n <= 34
+
+// sums of |a|^2 over 16 loads: total, and the four load bits' sums (added to acc)
+__device__ __forceinline__ double tree16(const double (&u)[16], double (&bit)[4]) {
+    double a[8], b[4], c[2];
 #pragma unroll
-    for (int q = 0; q < 17; q++) hb[q] = 0.0;
-    // it = (g << 4) | k: the 16 values of k are summed per bit in registers, group totals feed the
-    // bits above
-    const int ng = niter >= 16 ? niter >> 4 : 1;
-    const int gk = niter >= 16 ? 16 : niter;
-    for (int g = 0; g < ng; g++) {
+    for (int k = 0; k < 8; k++) a[k] = u[2 * k] + u[2 * k + 1];
+#pragma unroll
+    for (int k = 0; k < 4; k++) b[k] = a[2 * k] + a[2 * k + 1];
+    c[0] = b[0] + b[1];
+    c[1] = b[2] + b[3];
+    bit[0] += ((u[1] + u[3]) + (u[5] + u[7])) + ((u[9] + u[11]) + (u[13] + u[15]));
+    bit[1] += (a[1] + a[3]) + (a[5] + a[7]);
+    bit[2] += b[1] + b[3];
+    bit[3] += c[1];
+    return c[0] + c[1];
+}
+__device__ __forceinline__ double prob(float x, float y) { return (double)x * x + (double)y * y; }
+
+// 16 bytes of the state: two complex64 amplitudes or one complex128. AL: the state starts on a 16-byte boundary
+// (a view of a larger tensor may start between two)
+template <bool AL>
+__device__ __forceinline__ float4 load16(const float2 *p, int64_t i) {
+    if (AL) return reinterpret_cast<const float4 *>(p)[i];
+    const float2 a = p[2 * i], b = p[2 * i + 1];
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <bool AL>
+__device__ __forceinline__ double2 load16(const double2 *p, int64_t i) { return p[i]; }
+
+struct RedAcc {
+    double tot, vec;               // vec: bit 0 of complex64 (in the vector) / the fifth load bit of complex128
+    double ld[4];
+};
+// one chunk of a thread: returns the thread's total over the chunk
+template <bool AL>
+__device__ __forceinline__ double red_chunk(const float2 *p, int t, RedAcc &r) {
+    float4 x[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) x[k] = load16<AL>(p, t + 256 * k);
+    double u[16], one = 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const double hi = prob(x[k].z, x[k].w);
+        one += hi;
+        u[k] = prob(x[k].x, x[k].y) + hi;
+    }
+    r.vec += one;
+    return tree16(u, r.ld);
+}
+template <bool AL>
+__device__ __forceinline__ double red_chunk(const double2 *p, int t, RedAcc &r) {
+    double sum[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        double2 x[16];
         double u[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            u[k] = 0.0;
-            if (k < gk) {
-                const A a = state[base + t + ((int64_t)((g << 4) | k) << 8)];
-                u[k] = (double)a.x * a.x + (double)a.y * a.y;
-            }
-        }
-        double gt = 0.0;
+        for (int k = 0; k < 16; k++) x[k] = p[t + 256 * (16 * h + k)];
 #pragma unroll
-        for (int k = 0; k < 16; k++) gt += u[k];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            double s = 0.0;
-#pragma unroll
-            for (int k = 0; k < 16; k++)
-                if ((k >> q) & 1) s += u[k];
-            hb[q] += s;
-        }
-        for (int q = 4; q < B - 8; q++)
-            if ((g >> (q - 4)) & 1) hb[q] += gt;
-        tot += gt;
+        for (int k = 0; k < 16; k++) u[k] = x[k].x * x[k].x + x[k].y * x[k].y;
+        sum[h] = tree16(u, r.ld);
     }
-    s_tot[t] = tot;
-    for (int q = 0; q < 17; q++) s_bits[t][q] = hb[q];
+    r.vec += sum[1];
+    return sum[0] + sum[1];
+}
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Block b takes chunks b, b + gridDim.x, ...; out: nout doubles per block, the total and the sums of index bits
+// 0 .. nout - 2 (nout = 14: the bits of one chunk, or n + 1: all bits).
+template <class A, bool AL>
+__global__ void __launch_bounds__(RED_THREADS, 2)
+    reduce_chunks_kernel(const A *__restrict__ state, int64_t nchunks, int nout, double *__restrict__ partials) {
+    constexpr bool C64 = sizeof(A) == 8;
+    __shared__ double part[RED_THREADS / 32][RED_CHUNK_BITS + 1 + RED_HI];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    RedAcc r = {0.0, 0.0, {0.0, 0.0, 0.0, 0.0}};
+    double hi[RED_HI];
+#pragma unroll
+    for (int q = 0; q < RED_HI; q++) hi[q] = 0.0;
+    for (int64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const double s = red_chunk<AL>(state + (c << RED_CHUNK_BITS), t, r);
+        r.tot += s;
+        if (nout > RED_CHUNK_BITS + 1) {
+#pragma unroll
+            for (int q = 0; q < RED_HI; q++)
+                if ((c >> q) & 1) hi[q] += s;
+        }
+    }
+    auto put = [&](int o, double v) {
+        v = warp_sum(v);
+        if (lane == 0) part[warp][o] = v;
+    };
+    constexpr int T0 = C64 ? 1 : 0;              // first thread bit
+    put(0, r.tot);
+    if (C64) put(1, r.vec);
+#pragma unroll
+    for (int q = 0; q < 8; q++) put(1 + T0 + q, (t >> q) & 1 ? r.tot : 0.0);
+#pragma unroll
+    for (int q = 0; q < 4; q++) put(1 + T0 + 8 + q, r.ld[q]);
+    if (!C64) put(13, r.vec);
+    if (nout > RED_CHUNK_BITS + 1) {
+#pragma unroll
+        for (int q = 0; q < RED_HI; q++)
+            if (q < nout - 1 - RED_CHUNK_BITS) put(1 + RED_CHUNK_BITS + q, hi[q]);
+    }
     __syncthreads();
-    double *out = partials + (int64_t)blockIdx.x * (B + 1);
-    if (t == 0) {
+    if (t < nout) {
         double s = 0.0;
-        for (int i = 0; i < RED_THREADS; i++) s += s_tot[i];
-        out[0] = s;
-    } else if (t <= B) {
-        const int q = t - 1;        // index bit q
-        double s = 0.0;
-        if (q < 8) {
-            for (int i = 0; i < RED_THREADS; i++)
-                if ((i >> q) & 1) s += s_tot[i];
-        } else {
-            for (int i = 0; i < RED_THREADS; i++) s += s_bits[i][q - 8];
-        }
-        out[1 + q] = s;
+#pragma unroll
+        for (int w = 0; w < RED_THREADS / 32; w++) s += part[w][t];
+        partials[(int64_t)blockIdx.x * nout + t] = s;
     }
 }
 
-// out[0] = total, out[1 + q] = total - 2 * (sum over i with bit q set)
-__global__ void reduce_final_kernel(const double *__restrict__ partials, int nblocks, int B, int n,
-                                    double *__restrict__ out) {
-    const int t = threadIdx.x;
-    if (t > n) return;
+// states of fewer than 2^13 amplitudes: one block, a strided pass per output (nout = n + 1)
+template <class A>
+__global__ void __launch_bounds__(RED_THREADS)
+    reduce_small_kernel(const A *__restrict__ state, int n, double *__restrict__ partials) {
+    __shared__ double part[RED_THREADS / 32][RED_CHUNK_BITS + 1];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    double s[RED_CHUNK_BITS + 1];
+#pragma unroll
+    for (int q = 0; q <= RED_CHUNK_BITS; q++) s[q] = 0.0;
+    for (int i = t; i < (1 << n); i += RED_THREADS) {
+        const A a = state[i];
+        const double p = (double)a.x * a.x + (double)a.y * a.y;
+        s[0] += p;
+#pragma unroll
+        for (int q = 0; q < RED_CHUNK_BITS; q++)
+            if ((i >> q) & 1) s[1 + q] += p;
+    }
+#pragma unroll
+    for (int q = 0; q <= RED_CHUNK_BITS; q++) {
+        const double v = warp_sum(s[q]);
+        if (lane == 0) part[warp][q] = v;
+    }
+    __syncthreads();
+    if (t <= n) {
+        double v = 0.0;
+        for (int w = 0; w < RED_THREADS / 32; w++) v += part[w][t];
+        partials[t] = v;
+    }
+}
+
+// out[0] = total, out[1 + q] = total - 2 * (sum over i with bit q set). Block o reduces output o over the block
+// partials (nout each); with one-chunk partials (nout = 14) a bit above a chunk is a bit of the block number.
+__global__ void __launch_bounds__(128)
+    reduce_final_kernel(const double *__restrict__ partials, int nblocks, int nout, double *__restrict__ out) {
+    __shared__ double s_tot[4], s_bit[4];
+    const int o = blockIdx.x, t = threadIdx.x;
     double tot = 0.0, s = 0.0;
-    for (int b = 0; b < nblocks; b++) {
-        const double *p = partials + (int64_t)b * (B + 1);
-        tot += p[0];
-        if (t >= 1) {
-            const int q = t - 1;
-            if (q < B) s += p[1 + q];
-            else if ((b >> (q - B)) & 1) s += p[0];
-        }
+    for (int b = t; b < nblocks; b += 128) {
+        const double *p = partials + (int64_t)b * nout;
+        const double x = p[0];
+        tot += x;
+        if (o >= 1) s += o < nout ? p[o] : ((b >> (o - nout)) & 1 ? x : 0.0);
     }
-    if (t == 0) out[0] = tot;
-    else out[t] = tot - 2.0 * s;
+    tot = warp_sum(tot);
+    s = warp_sum(s);
+    if ((t & 31) == 0) { s_tot[t >> 5] = tot; s_bit[t >> 5] = s; }
+    __syncthreads();
+    if (t == 0) {
+        tot = (s_tot[0] + s_tot[1]) + (s_tot[2] + s_tot[3]);
+        s = (s_bit[0] + s_bit[1]) + (s_bit[2] + s_bit[3]);
+        out[o] = o == 0 ? tot : tot - 2.0 * s;
+    }
 }
 
-// chunk probabilities: one block per chunk of 2^cb amplitudes
+// ---------------------------------------------------------------- chunk probabilities
+// One warp per chunk of 2^cb amplitudes (cb >= CHUNK_WARP_MIN): 16-byte loads, eight in flight per lane, no block
+// barriers. Grid-strided over the chunks.
+#define CHUNK_WARP_MIN 8           // 256 complex64 amplitudes: 4 loads per lane
+#define CHUNK_WARP_MAX 13
+__device__ __forceinline__ double prob16(const float4 &v) { return prob(v.x, v.y) + prob(v.z, v.w); }
+__device__ __forceinline__ double prob16(const double2 &v) { return v.x * v.x + v.y * v.y; }
+template <class A, bool AL>
+__global__ void __launch_bounds__(RED_THREADS)
+    chunk_probs_warp_kernel(const A *__restrict__ state, int cb, int64_t nchunks, double *__restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t)gridDim.x * (RED_THREADS / 32);
+    const int len = (int)(((size_t)sizeof(A) << cb) / 16);       // a multiple of 128
+    for (int64_t c = (int64_t)blockIdx.x * (RED_THREADS / 32) + (threadIdx.x >> 5); c < nchunks; c += nw) {
+        const A *p = state + (c << cb);
+        double acc = 0.0;
+        int i = lane;
+        for (; i + 224 < len; i += 256) {
+            decltype(load16<AL>(p, 0)) v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = load16<AL>(p, i + 32 * k);
+#pragma unroll
+            for (int k = 0; k < 8; k++) acc += prob16(v[k]);
+        }
+        for (; i < len; i += 32) acc += prob16(load16<AL>(p, i));
+        acc = warp_sum(acc);
+        if (lane == 0) out[c] = acc;
+    }
+}
+
+// one block per chunk (any other chunk size)
 template <class A>
 __global__ void __launch_bounds__(RED_THREADS)
     chunk_probs_kernel(const A *__restrict__ state, int cb, double *__restrict__ out) {
     __shared__ double s[RED_THREADS];
     const int64_t base = (int64_t)blockIdx.x << cb;
-    const int len = 1 << cb;
+    const int64_t len = 1ll << cb;
     double acc = 0.0;
-    for (int i = threadIdx.x; i < len; i += RED_THREADS) {
+    for (int64_t i = threadIdx.x; i < len; i += RED_THREADS) {
         const A a = state[base + i];
         acc += (double)a.x * a.x + (double)a.y * a.y;
     }
@@ -263,60 +391,130 @@ __global__ void __launch_bounds__(RED_THREADS)
     if (threadIdx.x == 0) out[blockIdx.x] = s[0];
 }
 
-// inclusive prefix sum of nc doubles in one block (sequential per thread slice, fixed order)
-__global__ void scan_kernel(double *__restrict__ v, int64_t nc) {
-    __shared__ double part[1024];
-    const int t = threadIdx.x, nt = blockDim.x;
-    const int64_t per = (nc + nt - 1) / nt;
-    const int64_t b = t * per, e = b + per < nc ? b + per : nc;
-    double s = 0.0;
-    for (int64_t i = b; i < e; i++) s += v[i];
-    part[t] = s;
+// ---------------------------------------------------------------- Born sampler
+// Chunk probabilities are scanned in groups of 2^SCAN_BITS (one block each, in place), and the groups' totals by
+// every sampling block for itself: the cumulative sum up to chunk c is the total of the groups before c's plus
+// the scanned value. One warp per shot then finds the chunk (binary searches), the 1/32 of the chunk and the
+// amplitude, each the first whose running FP64 sum exceeds what is left of the draw.
+// What bounds it: the read of the state for the chunk probabilities. A scan of 2^16 values in one block and one
+// thread per shot adding up to 4096 amplitudes one after the other took 1.20 ms for 1024 shots of 28 qubits
+// (HBM floor 0.33 ms); now 0.36 ms, and 38 instead of 440-530 us at 12-20 qubits.
+#define SCAN_BITS 12
+#define SCAN_THREADS 1024
+__device__ __forceinline__ double warp_scan(double v, int lane) {       // inclusive
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += x;
+    }
+    return v;
+}
+__global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(double *__restrict__ v, int64_t nc) {
+    __shared__ double wsum[32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int64_t i = ((int64_t)blockIdx.x << SCAN_BITS) + 4 * t;
+    double x[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = i + k < nc ? v[i + k] : 0.0;
+    x[1] += x[0]; x[2] += x[1]; x[3] += x[2];
+    const double incl = warp_scan(x[3], lane);
+    if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    if (t == 0) {
+    if (warp == 0) wsum[lane] = warp_scan(wsum[lane], lane);
+    __syncthreads();
+    double before = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) before = 0.0;
+    if (warp > 0) before += wsum[warp - 1];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (i + k < nc) v[i + k] = before + x[k];
+}
+
+#define SAMPLE_WARPS 8
+#define SAMPLE_GROUPS 1024         // groups of chunks: 2^(34 - 12 - SCAN_BITS)
+template <class A>
+__global__ void __launch_bounds__(32 * SAMPLE_WARPS)
+    sample_kernel(const A *__restrict__ state, int cb, const double *__restrict__ cdf, int64_t nc,
+                  const double *__restrict__ uni, int shots, int64_t *__restrict__ out) {
+    __shared__ double gcdf[SAMPLE_GROUPS];       // inclusive sums of the group totals
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int ng = (int)((nc + (1 << SCAN_BITS) - 1) >> SCAN_BITS);
+    for (int g = t; g < ng; g += 32 * SAMPLE_WARPS) {
+        const int64_t last = ((int64_t)(g + 1) << SCAN_BITS) - 1;
+        gcdf[g] = cdf[last < nc ? last : nc - 1];
+    }
+    __syncthreads();
+    if (warp == 0) {
         double run = 0.0;
-        for (int i = 0; i < nt; i++) {
-            const double x = part[i];
-            part[i] = run;
-            run += x;
+        for (int g0 = 0; g0 < ng; g0 += 32) {
+            const double v = warp_scan(g0 + lane < ng ? gcdf[g0 + lane] : 0.0, lane) + run;
+            run = __shfl_sync(0xffffffffu, v, 31);
+            if (g0 + lane < ng) gcdf[g0 + lane] = v;
         }
     }
     __syncthreads();
-    double run = part[t];
-    for (int64_t i = b; i < e; i++) {
-        run += v[i];
-        v[i] = run;
-    }
-}
-
-// one thread per shot: chunk by binary search on the FP64 chunk cdf, then a linear FP64 scan inside
-// the chunk (first index whose running sum exceeds the remainder, clipped to the chunk)
-template <class A>
-__global__ void sample_kernel(const A *__restrict__ state, int cb, const double *__restrict__ cdf, int64_t nc,
-                              const double *__restrict__ uni, int shots, int64_t *__restrict__ out) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = blockIdx.x * SAMPLE_WARPS + warp;
     if (s >= shots) return;
-    const double total = cdf[nc - 1];
-    const double x = uni[s] * total;
-    int64_t lo = 0, hi = nc;        // first c with cdf[c] > x
+    const double x = uni[s] * gcdf[ng - 1];
+    int lo = 0, hi = ng;                         // first group whose cumulative sum exceeds x
     while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (cdf[mid] > x) hi = mid;
+        const int mid = (lo + hi) >> 1;
+        if (gcdf[mid] > x) hi = mid;
         else lo = mid + 1;
     }
-    int64_t c = lo < nc ? lo : nc - 1;
-    const double rem = x - (c > 0 ? cdf[c - 1] : 0.0);
-    const int len = 1 << cb;
-    const A *p = state + (c << cb);
-    double run = 0.0;
-    int j = 0;
-    for (; j < len; j++) {
-        const A a = p[j];
-        run += (double)a.x * a.x + (double)a.y * a.y;
-        if (run > rem) break;
+    const int g = lo < ng ? lo : ng - 1;
+    double rem = x - (g > 0 ? gcdf[g - 1] : 0.0);
+    const int64_t first = (int64_t)g << SCAN_BITS;
+    const int cnt = (int)(nc - first < (1 << SCAN_BITS) ? nc - first : 1 << SCAN_BITS);
+    lo = 0; hi = cnt;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cdf[first + mid] > rem) hi = mid;
+        else lo = mid + 1;
     }
-    if (j >= len) j = len - 1;
-    out[s] = (c << cb) + j;
+    const int cc = lo < cnt ? lo : cnt - 1;
+    if (cc > 0) rem -= cdf[first + cc - 1];
+    const int64_t base = (first + cc) << cb;
+    const A *p = state + base;
+    // the lane sums of 32 consecutive runs of `per` amplitudes; picks the first run whose cumulative sum exceeds
+    // rem (-1: none) and leaves in rem what remains inside it
+    auto pick = [&](double v) -> int {
+        double run = 0.0;
+        for (int k = 0; k < 32; k++) {
+            const double y = __shfl_sync(0xffffffffu, v, k);
+            if (run + y > rem) {
+                rem -= run;
+                return k;
+            }
+            run += y;
+        }
+        return -1;
+    };
+    auto prob_at = [&](int i) -> double {
+        const A a = p[i];
+        return (double)a.x * a.x + (double)a.y * a.y;
+    };
+    int at = 0, len = 1 << cb;                   // the run the draw lies in: [at, at + len), len >= 1024 / 32
+    while (len > 32) {
+        const int per = len >> 5;
+        double v = 0.0;
+#pragma unroll 8
+        for (int i = 0; i < per; i++) v += prob_at(at + lane * per + i);
+        const int k = pick(v);
+        if (k < 0) break;                        // rounding left the draw beyond the run's sum: its last amplitude
+        at += k * per;
+        len = per;
+    }
+    if (len <= 32) {
+        const double v = lane < len ? prob_at(at + lane) : 0.0;
+        const int k = pick(v);
+        const unsigned some = __ballot_sync(0xffffffffu, v > 0.0);
+        if (k >= 0) at += k;
+        else at += some ? 31 - __clz((int)some) : len - 1;
+    } else {
+        at += len - 1;
+    }
+    if (lane == 0) out[s] = base + at;
 }
 
 }  // namespace dev
@@ -413,16 +611,44 @@ size_t reduce_scratch_bytes(int n, int chunk_bits) {
     return red > smp ? red : smp;
 }
 
-cudaError_t launch_reduce(const void *state, int n, int dtype, double *out, void *scratch, cudaStream_t stream) {
+// The block partials of a reduction: `blocks` blocks of nout doubles. Up to 2^9 chunks (n = 22) every chunk is a
+// block of its own with the sums of its 13 bits; above, a grid of four blocks per SM takes chunks in turn and
+// keeps the sums of all n bits, as many blocks as fit the scratch that reduce_scratch_bytes declares.
+static void reduce_grid(int n, int nsm, int64_t *blocks, int *nout) {
     const int B = reduce_bits(n);
-    const int nblocks = 1 << (n - B);
-    double *partials = (double *)scratch;
-    if (dtype) dev::reduce_block_kernel<double2><<<nblocks, RED_THREADS, 0, stream>>>((const double2 *)state, B, partials);
-    else dev::reduce_block_kernel<float2><<<nblocks, RED_THREADS, 0, stream>>>((const float2 *)state, B, partials);
+    const int64_t room = (1ll << (n - B)) * (B + 1);
+    if (n <= RED_CHUNK_BITS) { *blocks = 1; *nout = n + 1; return; }
+    if (n <= 22) { *blocks = 1ll << (n - RED_CHUNK_BITS); *nout = RED_CHUNK_BITS + 1; return; }
+    int64_t g = (int64_t)nsm * 4;
+    if (g > room / (n + 1)) g = room / (n + 1);
+    if (g > 1ll << (n - RED_CHUNK_BITS)) g = 1ll << (n - RED_CHUNK_BITS);
+    *blocks = g;
+    *nout = n + 1;
+}
+
+static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <class A>
+static cudaError_t launch_reduce_t(const A *state, int n, int nsm, double *out, double *partials, cudaStream_t stream) {
+    int64_t blocks;
+    int nout;
+    reduce_grid(n, nsm, &blocks, &nout);
+    if (n < RED_CHUNK_BITS) dev::reduce_small_kernel<A><<<1, RED_THREADS, 0, stream>>>(state, n, partials);
+    else if (aligned16(state))
+        dev::reduce_chunks_kernel<A, true><<<(unsigned)blocks, RED_THREADS, 0, stream>>>(
+            state, 1ll << (n - RED_CHUNK_BITS), nout, partials);
+    else
+        dev::reduce_chunks_kernel<A, false><<<(unsigned)blocks, RED_THREADS, 0, stream>>>(
+            state, 1ll << (n - RED_CHUNK_BITS), nout, partials);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    dev::reduce_final_kernel<<<1, 64, 0, stream>>>(partials, nblocks, B, n, out);
+    dev::reduce_final_kernel<<<(unsigned)(n + 1), 128, 0, stream>>>(partials, (int)blocks, nout, out);
     return cudaGetLastError();
+}
+
+cudaError_t launch_reduce(const void *state, int n, int dtype, double *out, void *scratch, int nsm, cudaStream_t stream) {
+    if (dtype) return launch_reduce_t((const double2 *)state, n, nsm, out, (double *)scratch, stream);
+    return launch_reduce_t((const float2 *)state, n, nsm, out, (double *)scratch, stream);
 }
 
 // ---------------------------------------------------------------- reduction without caller scratch
@@ -467,7 +693,7 @@ static cudaError_t noalloc_scratch_ptr(double **out) {
     return cudaSuccess;
 }
 
-cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *out, cudaStream_t stream,
+cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *out, int nsm, cudaStream_t stream,
                                   size_t *need) {
     const size_t doubles = (size_t)noalloc_partials(n);
     *need = doubles * sizeof(double);
@@ -475,34 +701,47 @@ cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *o
     double *scratch = nullptr;
     cudaError_t e = noalloc_scratch_ptr(&scratch);
     if (e != cudaSuccess) return e;
-    return launch_reduce(state, n, dtype, out, scratch, stream);
+    return launch_reduce(state, n, dtype, out, scratch, nsm, stream);
 }
 
-cudaError_t launch_chunk_probs(const void *state, int n, int dtype, int cb, double *out, cudaStream_t stream) {
-    const unsigned nc = (unsigned)(1ll << (n - cb));
-    if (dtype) dev::chunk_probs_kernel<double2><<<nc, RED_THREADS, 0, stream>>>((const double2 *)state, cb, out);
-    else dev::chunk_probs_kernel<float2><<<nc, RED_THREADS, 0, stream>>>((const float2 *)state, cb, out);
+template <class A>
+static cudaError_t launch_chunk_probs_t(const A *state, int n, int cb, double *out, int nsm, cudaStream_t stream) {
+    const int64_t nc = 1ll << (n - cb);
+    if (cb >= CHUNK_WARP_MIN && cb <= CHUNK_WARP_MAX) {
+        int64_t grid = (nc + RED_THREADS / 32 - 1) / (RED_THREADS / 32);
+        if (grid > (int64_t)nsm * 8) grid = (int64_t)nsm * 8;
+        if (aligned16(state))
+            dev::chunk_probs_warp_kernel<A, true><<<(unsigned)grid, RED_THREADS, 0, stream>>>(state, cb, nc, out);
+        else
+            dev::chunk_probs_warp_kernel<A, false><<<(unsigned)grid, RED_THREADS, 0, stream>>>(state, cb, nc, out);
+    } else {
+        dev::chunk_probs_kernel<A><<<(unsigned)nc, RED_THREADS, 0, stream>>>(state, cb, out);
+    }
     return cudaGetLastError();
 }
 
+cudaError_t launch_chunk_probs(const void *state, int n, int dtype, int cb, double *out, int nsm, cudaStream_t stream) {
+    if (dtype) return launch_chunk_probs_t((const double2 *)state, n, cb, out, nsm, stream);
+    return launch_chunk_probs_t((const float2 *)state, n, cb, out, nsm, stream);
+}
+
 cudaError_t launch_sample(const void *state, int n, int dtype, int cb, const double *uni, int shots, int64_t *out,
-                          void *scratch, cudaStream_t stream) {
+                          void *scratch, int nsm, cudaStream_t stream) {
     double *cdf = (double *)scratch;
     const int64_t nc = 1ll << (n - cb);
-    cudaError_t e0 = launch_chunk_probs(state, n, dtype, cb, cdf, stream);
-    if (e0 != cudaSuccess) return e0;
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chunk_probs(state, n, dtype, cb, cdf, nsm, stream);
     if (e != cudaSuccess) return e;
-    dev::scan_kernel<<<1, 1024, 0, stream>>>(cdf, nc);
+    dev::scan_kernel<<<(unsigned)((nc + (1 << SCAN_BITS) - 1) >> SCAN_BITS), SCAN_THREADS, 0, stream>>>(cdf, nc);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (shots > 0) {
+        const unsigned grid = (unsigned)((shots + SAMPLE_WARPS - 1) / SAMPLE_WARPS);
         if (dtype)
-            dev::sample_kernel<double2><<<(shots + 127) / 128, 128, 0, stream>>>((const double2 *)state, cb, cdf, nc, uni,
-                                                                                 shots, out);
-        else
-            dev::sample_kernel<float2><<<(shots + 127) / 128, 128, 0, stream>>>((const float2 *)state, cb, cdf, nc, uni,
+            dev::sample_kernel<double2><<<grid, 32 * SAMPLE_WARPS, 0, stream>>>((const double2 *)state, cb, cdf, nc, uni,
                                                                                 shots, out);
+        else
+            dev::sample_kernel<float2><<<grid, 32 * SAMPLE_WARPS, 0, stream>>>((const float2 *)state, cb, cdf, nc, uni,
+                                                                               shots, out);
     }
     return cudaGetLastError();
 }
