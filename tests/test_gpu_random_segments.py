@@ -6,7 +6,8 @@ import sys
 import numpy as np
 import pytest
 
-from qsv_b200 import engine
+from qsv_b200 import compile_circuit, engine
+from qsv_b200.generators import random_layer
 from oracle import oracle as orc
 
 sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
@@ -35,5 +36,31 @@ def test_random_segments_exact(shape, dtype):
             assert engine.device_status() == 0
             ref = orc.run_segment(x.copy(), seg)
             assert np.array_equal(t.cpu().numpy(), ref), f"n={n} k={k} seed={seed}"
+    finally:
+        engine.set_jit(old)
+
+
+@pytest.mark.parametrize("mode", ["eager", "coarse"])
+@pytest.mark.parametrize("shape", [(10, 10, 2, 20), (12, 12, 2, 20), (13, 12, 2, 20), (17, 9, 8, 6), (19, 12, 4, 8)])
+def test_random_segments_specialised_exact(shape, mode):
+    torch = pytest.importorskip("torch")
+    n, k, passes, ops = shape
+    segs = [random_segment(n, k, passes, ops, 7 * n)]
+    # one U3 (real first entry) on every qubit: targets in every slot, lane bits among them
+    layer, _, _ = compile_circuit(random_layer(n, 2, n), n, min(n, 12))
+    segs += [p for what, p in layer]
+    x = random_state(n, n)
+    old = engine.set_jit(mode)
+    try:
+        for seg in segs:
+            engine.jit_prepare(seg, n)
+            before = engine.jit_info()["jit_launches"]
+            t = torch.from_numpy(x.copy()).cuda()
+            engine.run_segment(t, seg)
+            torch.cuda.synchronize()
+            assert engine.device_status() == 0
+            assert engine.jit_info()["jit_launches"] > before
+            x = orc.run_segment(x.copy(), seg)
+            assert np.array_equal(t.cpu().numpy(), x)
     finally:
         engine.set_jit(old)

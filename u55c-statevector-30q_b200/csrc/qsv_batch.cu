@@ -32,7 +32,7 @@ namespace dev {
 template <int KW, int RB, int WB, int S>
 __global__ void __launch_bounds__((1 << (5 + WB)) + 32, (KW >= 13 ? 1 : 2))
     batch_kernel(const BatchItem *__restrict__ items, int nitems, const QsvPhaseX *__restrict__ phases,
-                 const QsvIOp *__restrict__ ops, int *status) {
+                 const QsvIOp *__restrict__ ops, uint32_t zero, int *status) {
     constexpr int NC = 1 << (5 + WB);
     constexpr int NV = 1 << RB;
     constexpr int TILE = 1 << KW;
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__((1 << (5 + WB)) + 32, (KW >= 13 ? 1 : 2))
         for (int ph = it.ph_begin; ph < it.ph_end; ph++) {
             if (ph > it.ph_begin) named_bar_sync(1, NC);
             const QsvPhaseX &Q = phases[ph];
-            run_phase<NV, RB, WB>(tile, Q, ops, Q.op_begin, Q.op_end, lane, warp, false, ph > it.ph_begin,
+            run_phase<NV, RB, WB>(tile, Q, ops, Q.op_begin, Q.op_end, lane, warp, zero, false, ph > it.ph_begin,
                                   ph + 1 < it.ph_end);
         }
         fence_proxy_async_smem();
@@ -113,7 +113,7 @@ static cudaError_t launch_batch_t(const BatchItem *items, int nitems, const QsvP
     }
     int64_t grid = (int64_t)nsm * per_sm;
     if (grid > nitems) grid = nitems;
-    batch_kernel<KW, RB, WB, S><<<(unsigned)grid, NT, smem, stream>>>(items, nitems, phases, ops, status);
+    batch_kernel<KW, RB, WB, S><<<(unsigned)grid, NT, smem, stream>>>(items, nitems, phases, ops, 0u, status);
     return cudaGetLastError();
 }
 

@@ -46,6 +46,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "qsv_iop.h"
 #include "qsv_planner.h"
 #include "_gen/qsv_jit_headers.inc"
 
@@ -93,16 +94,6 @@ int groups_for(const QsvSweep &sw, int wb) {
 // 0.5-2 % faster and the FP32-bound sweeps over qubits 0-12 5-15 % slower (their prefetch depth drops from
 // two tiles to one). QSV_JIT_INTERLEAVE=1: multi-phase tensor-map sweeps of one consumer group; =2: every
 // multi-phase sweep of one consumer group.
-// Whether uncontrolled dense ops on register bits use the coefficient-major form (jit_reg_cm). Tuning
-// switch QSV_JIT_CM=1; off by default.
-bool coef_major() {
-    static const bool on = [] {
-        const char *e = std::getenv("QSV_JIT_CM");
-        return e && std::atoi(e) == 1;
-    }();
-    return on;
-}
-
 int interleave_for(const QsvSweep &sw, int groups) {
     static const int mode = [] {
         const char *e = std::getenv("QSV_JIT_INTERLEAVE");
@@ -380,10 +371,36 @@ std::string gen_source_lib(const std::vector<std::string> &types, int rb, int wb
     return s.str();
 }
 
+// Coefficients a specialised kernel reads for an op: none for exchanges, 12 for one matrix, 24 for a choice of two.
+int coef_count(const QsvOp &op) {
+    if (op.variant == QSV_V_SKIP || is_swap_variant(op.variant)) return 0;
+    return op.kind == QSV_K_MUX ? 24 : 12;
+}
+int coef_total(const QsvSweep &sw) {
+    int n = 0;
+    for (int o = 0; o < sw.nops; o++) n += coef_count(sw.ops[o]);
+    return n > 0 ? n : 1;
+}
+// what a specialised kernel is given (QsvSweepJ; the kernel's parameter holds as many coefficients as it reads)
+struct JitParams : QsvSweepHead {
+    unsigned long long coef[24 * QSV_MAX_SWEEP_OPS];
+};
+static_assert(sizeof(QsvSweepHead) == sizeof(QsvSweepJ<2>) - 16, "coefficients follow the head");
+void jit_params(const QsvSweep &sw, JitParams &P) {
+    static_cast<QsvSweepHead &>(P) = sw;
+    int at = 0;
+    for (int o = 0; o < sw.nops; o++) {
+        const int n = coef_count(sw.ops[o]);
+        for (int e = 0; e < n; e++) P.coef[at + e] = dev::iop_coef(sw.ops[o], e);
+        at += n;
+    }
+}
+
 // CUDA source of the kernel specialised to sw's structure
 std::string gen_source(const QsvSweep &sw, int rb, int wb) {
     const int groups = groups_for(sw, wb);
     const int nc = 1 << (5 + wb), nt = groups * nc + 32, minb = sw.kw >= 13 ? 1 : 2;
+    const std::string param = "QsvSweepJ<" + std::to_string(coef_total(sw)) + ">";
     std::ostringstream s;
     s << "#include \"qsv_sweep_body.cuh\"\n#include \"qsv_jit_ops.cuh\"\n"
       << "namespace qsv {\nnamespace dev {\nstruct JitBody {\n"
@@ -393,58 +410,57 @@ std::string gen_source(const QsvSweep &sw, int rb, int wb) {
       << "    static constexpr int kPhases = " << sw.nphases << ";\n"
       << "    // one phase of a tile: load in the phase's layout, apply its ops, store\n"
       << "    template <int NV, int RB, int WB>\n"
-      << "    static __device__ __forceinline__ void phase(int p, float2 *tile, const QsvSweep &P, const QsvOp *, int lane,\n"
-      << "                                                 int warp) {\n"
+      << "    static __device__ __forceinline__ void phase(int p, float2 *tile, const " << param << " &P, const QsvOp *,\n"
+      << "                                                 int lane, int warp) {\n"
+      << "        const p2 *C = P.coef;\n"
       << "        switch (p) {\n";
+    int coef_at = 0;
     for (int p = 0; p < sw.nphases; p++) {
         const QsvPhase &ph = sw.phases[p];
         s << "        case " << p << ": {\n            const uint32_t tb = jit_lane_base<" << (int)ph.lane_lo[0] << ", "
           << (int)ph.lane_lo[1] << ", " << (int)ph.lane_lo[2] << ", " << (int)ph.lane_bits[0] << ", "
           << (int)ph.lane_bits[1] << ">(lane)";
         for (int w = 0; w < wb; w++) s << " | jit_warp_bit<" << (int)ph.warp_bits[w] << ">(warp, " << w << ")";
-        s << ";\n            float2 R[NV], I[NV];\n";
+        s << ";\n            p2 R[NV], I[NV];\n";
         std::string rbits;
         for (int r = 0; r < rb; r++) rbits += (r ? ", " : "") + std::to_string((int)ph.reg_bits[r]);
         s << "            jit_load<NV, " << (int)sw.swz << ", " << (p > 0 ? 1 : 0) << ", " << rbits
-          << ">(tile, tb, R, I);\n";
+          << ">(tile, tb, P.zero, R, I);\n";
         for (int o = ph.op_begin; o < ph.op_end; o++) {
             const QsvOp &op = sw.ops[o];
+            const int at = coef_at;
+            coef_at += coef_count(op);
+            if (op.variant == QSV_V_SKIP) continue;
             const std::string thr = std::to_string(op.cm_thr) + "u";
             // m00-real dense ops take the QSV_M_DENSE_R0 / QSV_V_UNI_DENSE_R0 code paths
             const bool r0 = op.r00 && op.kind == QSV_K_UNI;
             const int cls0 = r0 ? QSV_M_DENSE_R0 : op.cls0;
             const int var = (r0 && op.variant == QSV_V_UNI_DENSE) ? QSV_V_UNI_DENSE_R0 : op.variant;
-            const std::string cls = std::to_string((int)op.kind) + ", " + std::to_string(cls0) + ", " +
-                                    std::to_string((int)op.cls1) + ", ";
             const std::string ctl = std::to_string((int)op.cm_reg) + ", " + thr;
-            const std::string mux = std::to_string((int)op.kind) + ", " + std::to_string((int)op.cls1) + ", " +
-                                    std::to_string((int)op.cm_c) + ", " + ctl;
+            const std::string cls = std::to_string((int)op.kind) + ", " + std::to_string(cls0) + ", " +
+                                    std::to_string((int)op.cls1) + ", " + ctl;
+            const std::string mux = std::to_string((int)op.kind) + ", " + std::to_string((int)op.cls1) + ", " + ctl;
+            const int plain_var = op.slot < QSV_SLOT_LANE0 ? var : op.variant;     // (lane ops have no such form)
+            const std::string plain = std::to_string(plain_var) + ", " + std::to_string((int)op.cls0) + ", " + ctl;
+            const std::string args = ">(R, I, C + " + std::to_string(at) + ", tb";
             if (op.slot == QSV_SLOT_COMP)
-                s << "            jit_comp<NV, " << cls << ctl << ">(R, I, P.ops[" << o << "], tb);\n";
+                s << "            jit_comp<NV, " << cls << args << ");\n";
             else if (op.slot < QSV_SLOT_LANE0 && op.variant == QSV_V_MUX)
-                s << "            jit_reg_mux<NV, " << (op.slot - QSV_SLOT_REG0) << ", " << mux << ">(R, I, P.ops[" << o
-                  << "], tb);\n";
-            else if (op.slot < QSV_SLOT_LANE0 && coef_major() &&
-                     (var == QSV_V_UNI_DENSE || var == QSV_V_UNI_DENSE_R0))
-                s << "            jit_reg_cm<NV, " << (op.slot - QSV_SLOT_REG0) << ", " << var << ">(R, I, P.ops[" << o
-                  << "]);\n";
+                s << "            jit_reg_mux<NV, " << (op.slot - QSV_SLOT_REG0) << ", " << mux << args << ");\n";
             else if (op.slot < QSV_SLOT_LANE0)
-                s << "            jit_reg<NV, " << (op.slot - QSV_SLOT_REG0) << ", " << var << ", " << ctl
-                  << ">(R, I, P.ops[" << o << "], tb);\n";
+                s << "            jit_reg<NV, " << (op.slot - QSV_SLOT_REG0) << ", " << plain << args << ");\n";
             else if (op.variant == QSV_V_MUX)
-                s << "            jit_lane_mux<NV, " << (op.slot - QSV_SLOT_LANE0) << ", " << mux << ">(R, I, P.ops["
-                  << o << "], tb, lane);\n";
+                s << "            jit_lane_mux<NV, " << (op.slot - QSV_SLOT_LANE0) << ", " << mux << args << ", lane);\n";
             else
-                s << "            jit_lane<NV, " << (op.slot - QSV_SLOT_LANE0) << ", " << (int)op.variant << ", " << ctl
-                  << ">(R, I, P.ops[" << o << "], tb, lane);\n";
+                s << "            jit_lane<NV, " << (op.slot - QSV_SLOT_LANE0) << ", " << plain << args << ", lane);\n";
         }
         s << "            jit_store<NV, " << (int)sw.swz << ", " << (p + 1 < sw.nphases ? 1 : 0) << ", " << rbits
-          << ">(tile, tb, R, I);\n            break;\n        }\n";
+          << ">(tile, tb, P.zero, R, I);\n            break;\n        }\n";
     }
     s << "        default: break;\n        }\n    }\n"
       << "    template <int NV, int RB, int WB>\n"
-      << "    static __device__ __forceinline__ void tile(float2 *tile, const QsvSweep &P, const QsvOp *ops, int lane, int warp,\n"
-      << "                                                int bar) {\n"
+      << "    static __device__ __forceinline__ void tile(float2 *tile, const " << param << " &P, const QsvOp *ops, int lane,\n"
+      << "                                                int warp, int bar) {\n"
       << "#pragma unroll\n"
       << "        for (int p = 0; p < kPhases; p++) {\n"
       << "            if (p > 0) named_bar_sync(bar, " << nc << ");\n"
@@ -452,10 +468,10 @@ std::string gen_source(const QsvSweep &sw, int rb, int wb) {
       << "        }\n    }\n";
     s << "};\n}  // namespace dev\n}  // namespace qsv\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << nt << ", " << minb << ")\n"
-      << "    qsv_sweep_jit(float2 *__restrict__ state, const __grid_constant__ QsvSweep P,\n"
+      << "    qsv_sweep_jit(float2 *__restrict__ state, const __grid_constant__ " << param << " P,\n"
       << "                  const __grid_constant__ CUtensorMap tmap, int *status) {\n"
       << "    qsv::dev::sweep_pipeline<" << sw.kw << ", " << rb << ", " << wb << ", " << kStages << ", " << groups
-      << ", qsv::dev::JitBody, QsvSweep, " << interleave_for(sw, groups) << ">(state, P, &tmap, status);\n}\n";
+      << ", qsv::dev::JitBody, " << param << ", " << interleave_for(sw, groups) << ">(state, P, &tmap, status);\n}\n";
     return s.str();
 }
 
@@ -997,7 +1013,13 @@ int jit_try_launch(float2 *state, const QsvSweep &sw_in, int nsm, cudaStream_t s
     if (ce != cudaSuccess) { *err = ce; return -1; }
     int64_t grid = (int64_t)nsm * e->per_sm[dev];
     if (grid > sw.ntiles) grid = sw.ntiles;
-    void *args[] = {&state, const_cast<QsvSweep *>(lp), &map, &status};
+    thread_local JitParams jp;
+    void *param = const_cast<QsvSweep *>(lp);
+    if (!e->stream) {
+        jit_params(e->coarse ? coarse_of(*lp) : *lp, jp);
+        param = &jp;
+    }
+    void *args[] = {&state, param, &map, &status};
     if (d.launch(e->fn[dev], (unsigned)grid, 1, 1, (unsigned)NT, 1, 1, (unsigned)smem, (CUstream)stream, args,
                  nullptr) != CUDA_SUCCESS) {
         *err = cudaErrorLaunchFailure;

@@ -161,9 +161,8 @@ struct QsvGroup {
     int16_t type;               // group-type library: case of this group's op sequence (-1: none)
 };
 
-template <class OpT>
-struct QsvSweepT {
-    typedef OpT op_type;
+// What the staging pipeline reads of a sweep, whatever its ops.
+struct alignas(16) QsvSweepHead {
     int32_t n;                  // state qubits
     int32_t kw;                 // window size (tile = 2^kw amplitudes)
     int32_t lo;                 // contiguous low bits of the window
@@ -184,11 +183,25 @@ struct QsvSweepT {
     int32_t nphases;
     int32_t nops;
     uint32_t wait_us;           // bounded waits give up after this many microseconds (0: QSV_WAIT_US_DEFAULT)
+    uint32_t zero;              // 0, unknown to the compiler (see swap_mid in qsv_packed.cuh)
     int32_t skip_load;          // fault injection for tests: 1 = block 0 never loads its first tile (0: off)
+};
+
+template <class OpT>
+struct QsvSweepT : QsvSweepHead {
+    typedef OpT op_type;
     QsvPhase phases[QSV_MAX_PHASES];
     OpT ops[QSV_MAX_SWEEP_OPS];
     int32_t ngroups;            // streaming plan (plan_stream; 0 until planned)
     QsvGroup groups[QSV_MAX_GROUPS];
+};
+
+// Parameters of a kernel specialised to one sweep structure: its ops are code, only the NC coefficients they
+// read (packed, per op in order, see jit_coefs in qsv_jit.cpp) are data.
+template <int NC>
+struct QsvSweepJ : QsvSweepHead {
+    typedef QsvOp op_type;
+    unsigned long long coef[NC];
 };
 typedef QsvSweepT<QsvOp> QsvSweep;      // complex64 state, fp32 matrices
 typedef QsvSweepT<QsvOpD> QsvSweepD;    // complex128 state, fp64 matrices

@@ -61,7 +61,7 @@ struct InterpBody {
         for (int ph = 0; ph < P.nphases; ph++) {
             if (ph > 0) named_bar_sync(bar, NC);
             const QsvPhase &Q = P.phases[ph];
-            run_phase<NV, RB, WB>(tile, Q, iops, Q.op_begin, Q.op_end, lane, warp, P.swz != 0, ph > 0,
+            run_phase<NV, RB, WB>(tile, Q, iops, Q.op_begin, Q.op_end, lane, warp, P.zero, P.swz != 0, ph > 0,
                                   ph + 1 < P.nphases);
         }
     }
@@ -285,7 +285,7 @@ cudaError_t launch_sweep(float2 *state, const QsvSweep &sw_in, bool planned, int
     if (!planned && !interp_is_phase()) return launch_stream(state, sw_in, nsm, stream);
     thread_local QsvSweep own;
     if (!planned) {
-        std::memcpy(&own, &sw_in, offsetof(QsvSweep, ngroups));
+        own = sw_in;
         std::string err;
         if (plan_interp(own, err) != QSV_OK) return cudaErrorInvalidValue;
     }

@@ -129,7 +129,7 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
     __shared__ volatile int abort_flag;
 
     const int tid = threadIdx.x;
-    if (Body::kSmemOps) {
+    if constexpr (Body::kSmemOps) {
         const uint32_t *src = reinterpret_cast<const uint32_t *>(P.ops);
         uint32_t *dst = reinterpret_cast<uint32_t *>(sops);
         const int words = P.nops * (int)(sizeof(Op) / 4);
