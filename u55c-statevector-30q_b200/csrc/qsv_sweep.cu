@@ -21,6 +21,7 @@
 
 #include "qsv_device.cuh"
 #include "qsv_interp.cuh"
+#include "qsv_launch.h"
 #include "qsv_ops.cuh"
 #include "qsv_planner.h"
 #include "qsv_stream.cuh"
@@ -186,8 +187,7 @@ static cudaError_t launch_stream_t(float2 *state, const QsvSweep &sw, int nsm, c
     if (e != cudaSuccess) return e;
     int64_t grid = (int64_t)nsm * per_sm;
     if (grid > sw.ntiles) grid = sw.ntiles;
-    sweep_stream_kernel<KW, RB, WB, S, G, IP><<<(unsigned)grid, NT, smem, stream>>>(state, sw, map);
-    return cudaGetLastError();
+    return launch_behind(sweep_stream_kernel<KW, RB, WB, S, G, IP>, (unsigned)grid, NT, smem, stream, state, sw, map);
 }
 
 template <int KW, int RB, int WB, int S>
@@ -212,8 +212,7 @@ static cudaError_t launch_sweep_t(float2 *state, const QsvSweep &sw, int nsm, cu
     if (e != cudaSuccess) return e;
     int64_t grid = (int64_t)nsm * per_sm;
     if (grid > sw.ntiles) grid = sw.ntiles;
-    sweep_kernel<KW, RB, WB, S><<<(unsigned)grid, NT, smem, stream>>>(state, sw, map);
-    return cudaGetLastError();
+    return launch_behind(sweep_kernel<KW, RB, WB, S>, (unsigned)grid, NT, smem, stream, state, sw, map);
 }
 
 }  // namespace dev

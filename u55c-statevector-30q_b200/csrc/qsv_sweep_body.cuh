@@ -234,6 +234,9 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
         };
         Place ps, pl;
         int64_t issued = 0, j = 0;                    // loads issued for tiles [0, issued)
+        // Sweeps are launched behind one another (launch_behind): everything up to here, and the consumers' op
+        // expansion, overlaps the end of the sweep before; its state is read only after it.
+        grid_wait();
         for (; issued < S && issued < nmine; issued++) {
             place(issued, pl);
             issue_load(issued, (int)issued, pl);
@@ -244,6 +247,9 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
             place(j, ps);
             if (j + S < nmine) place(j + S, pl);
             if (!mbar_wait(&done[b], par, &abort_flag, status, limit)) break;
+            // the last tile's store is all that is left: the next sweep's blocks may come (earlier they would
+            // only hold their SMs, which sweeps on other streams can use)
+            if (j + 1 == nmine) grid_launch_dependents();
             issue_store(b, ps);
             if (j + S < nmine) {
                 bulk_wait_read_all();                 // this lane's stores have read the buffer

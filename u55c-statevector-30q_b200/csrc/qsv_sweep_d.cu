@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "qsv_device.cuh"
+#include "qsv_launch.h"
 #include "qsv_planner.h"
 #include "qsv_sweep_body.cuh"
 
@@ -342,8 +343,7 @@ static cudaError_t launch_c128_t(double2 *state, const QsvSweepD &sw, int nsm, i
     if (e != cudaSuccess) return e;
     int64_t grid = (int64_t)nsm * per_sm;
     if (grid > sw.ntiles) grid = sw.ntiles;
-    sweep_kernel_c128<KW, RB, WB, S><<<(unsigned)grid, NT, smem, stream>>>(state, sw, map, status);
-    return cudaGetLastError();
+    return launch_behind(sweep_kernel_c128<KW, RB, WB, S>, (unsigned)grid, NT, smem, stream, state, sw, map, status);
 }
 
 }  // namespace dev
