@@ -68,13 +68,20 @@ QSV_HD p2 pack2(float lo, float hi) {
 #endif
 }
 // a factor on the amplitudes with the target and every control set: diag(1, d), with or without controls
-QSV_HD bool iop_phase(const QsvOp &op) {
+template <class Op>
+QSV_HD bool iop_phase(const Op &op) {
     return op.variant == QSV_V_CTRL_DIAG1 || op.variant == QSV_V_CTRL_DIAG1_SEL ||
            (op.variant == QSV_V_MUX && op.kind == QSV_K_CTRL && op.cls1 == QSV_M_DIAG1) ||
            (op.variant == QSV_V_UNI_DIAG && op.cls == QSV_M_DIAG1);
 }
+// complex128: the same header and paths (no tile-bit-0 forms), the applied matrix and, for a choice of two, the other
+struct alignas(16) QsvIOpD {
+    uint32_t cm_thr, path, sel, aux;
+    double a[8], b[8];
+};
 // the header of an expanded record; slots: 2^(register bits) of the layout the op was planned for
-QSV_HD void iop_header(const QsvOp &op, int slots, QsvIOp &o) {
+template <class Op, class IOp>
+QSV_HD void iop_header(const Op &op, int slots, IOp &o) {
     const int slot = op.slot, v = op.variant;
     const bool lane = slot >= QSV_SLOT_LANE0, comp = slot == QSV_SLOT_COMP, base = slot == QSV_SLOT_BASE;
     const int rb = slot - QSV_SLOT_REG0;

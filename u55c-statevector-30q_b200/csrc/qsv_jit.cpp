@@ -67,13 +67,32 @@ constexpr size_t kMaxEntries = 8192;   // structures tracked; past it, the ones 
 constexpr int kMaxDevices = 64;
 constexpr int kStages = 3;         // tile buffers in flight (as the interpreter)
 
-// Consumer groups per CTA for a sweep. Two groups (16 consumer warps taking alternate tiles, registers
-// capped at 96 per thread: 17 warps share the four schedulers' register files) overlap one group's phase
-// round trips with the other's arithmetic. Warp-shuffle ops need the most registers: with more than three
-// the kernel spills, so it takes one group. Measured on the 30-qubit random-layer program: 3.05 -> 2.96 ms
-// for sweeps with 7-8 dense ops; with swizzled layouts, 4.65-4.69 -> 4.46-4.53 ms for the FP32-bound
-// sweeps with 12 dense ops and 0-3 shuffle ops (before swizzled layouts those had 5-6 shuffle ops and ran
-// slower with two groups, 4.4 -> 5.3 ms). QSV_JIT_GROUPS13=1 or 2 forces one choice.
+// Multiply-adds per amplitude of a sweep's ops as a specialised kernel runs them.
+double fma_work(const QsvSweep &sw) {
+    double w = 0.0;
+    for (int o = 0; o < sw.nops; o++) {
+        const QsvOp &op = sw.ops[o];
+        const double sel = 1.0 / (double)(1 << __builtin_popcount(op.cm_reg));    // other controls save no issue
+        switch (op.variant) {
+            case QSV_V_UNI_DENSE: w += op.r00 ? 7.0 : 8.0; break;
+            case QSV_V_UNI_DIAG: w += op.cls0 == QSV_M_DIAG1 ? 2.0 : 4.0; break;
+            case QSV_V_CTRL_DENSE: case QSV_V_CTRL_DENSE_SEL: w += 8.0 * sel; break;
+            case QSV_V_CTRL_DIAG1: case QSV_V_CTRL_DIAG1_SEL: w += 2.0 * sel; break;
+            case QSV_V_MUX: w += op.kind == QSV_K_MUX ? 8.0 : op.cls1 == QSV_M_DENSE ? 4.0 * sel : 1.0 * sel; break;
+            default: break;
+        }
+    }
+    return w;
+}
+
+// Consumer groups per CTA for a sweep. Two groups (16 consumer warps taking alternate tiles, registers capped at 96
+// per thread: 17 warps share the four schedulers' register files) overlap one group's phase round trips with the
+// other's arithmetic, but leave one of the three tile buffers for the copies; one group leaves two, which suits
+// sweeps of few ops, bound by HBM. Measured at 28 qubits (floor 656 us), one group / two: no or one dense op (up to
+// 24 multiply-adds per amplitude) 724 / 737 us and a transform of 45 sweeps 34.4 / 34.8 ms; 8 dense ops with real m00
+// (56) 672 / 687 us alone, but 262 / 260 ms for a 30-qubit circuit of such sweeps and 502 / 491 us at 22 qubits; 10
+// dense ops (72) 965 / 934, 12 in three phases (84) 922 / 846. Warp-shuffle ops need the most registers: with more
+// than three of them one group. QSV_JIT_GROUPS13=1 or 2 forces one choice.
 int groups_for(const QsvSweep &sw, int wb) {
     static const int forced = [] {
         const char *e = std::getenv("QSV_JIT_GROUPS13");
@@ -86,7 +105,7 @@ int groups_for(const QsvSweep &sw, int wb) {
         const QsvOp &op = sw.ops[o];
         lane += op.slot >= QSV_SLOT_LANE0 && op.variant != QSV_V_SKIP;
     }
-    return lane <= 3 ? 2 : 1;
+    return lane <= 3 && fma_work(sw) > 40.0 ? 2 : 1;
 }
 
 // Whether a sweep's kernel interleaves the phases of two tiles per consumer thread (sweep_pipeline IL).

@@ -137,8 +137,8 @@ int layout_interp(int kw, int *rb, int *wb) {
 
 int layout_for_kw_c128(int kw, int *rb, int *wb) {
     if (kw < 10 || kw > 12) return -1;
-    *rb = 4;
-    *wb = kw - 9;
+    *rb = 3;
+    *wb = kw - 8;
     return 0;
 }
 

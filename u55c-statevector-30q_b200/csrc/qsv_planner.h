@@ -44,7 +44,7 @@ int set_rb13(int rb);
 // How many of a phase's targets (tile bits >= 4) may sit on lane bits 3, 4 (0..2; default 1).
 int set_phase_lanes(int k);
 // Register/warp bit split of the complex128 layout for a window of kw qubits (kw in 10..12): tile bits
-// 0-2 on lane bits 0-2, two chosen lane bits, 4 register bits, kw - 9 warp bits.
+// 0-2 on lane bits 0-2, two chosen lane bits, 3 register bits, kw - 8 warp bits.
 int layout_for_kw_c128(int kw, int *rb, int *wb);
 // Merge consecutive passes into sweeps of window kw; merged windows keep >= 2^lo_merge contiguous amps.
 // OpT = QsvOp (complex64) or QsvOpD (complex128).

@@ -20,7 +20,9 @@
 #include <cuda_runtime.h>
 
 #include "qsv_device.cuh"
+#include "qsv_iop.h"
 #include "qsv_launch.h"
+#include "qsv_packed.cuh"
 #include "qsv_planner.h"
 #include "qsv_sweep_body.cuh"
 
@@ -33,10 +35,10 @@ __device__ __forceinline__ void lin_own_d(double &yr, double &yi, double ar, dou
     yi = fma(ar, owi, fma(ai, owr, fma(br, oti, __dmul_rn(bi, otr))));
 }
 
-// ---------------------------------------------------------------- ops by target slot
-// One uniform dispatch per op selects a tight loop over the thread's pairs, coefficients in registers. Each
-// loop computes the partial sums of all four outputs of a pair first and the final multiply-adds last, so
-// that every final is the last use of the input it replaces and can be written over its registers.
+// ---------------------------------------------------------------- ops by path (qsv_iop.h)
+// One tight loop over the thread's pairs per path. Each loop computes the partial sums of all four outputs of a pair
+// first and the final multiply-adds last, so that every final is the last use of the input it replaces and can be
+// written over its registers.
 struct MatD {
     double m[8];
 };
@@ -68,201 +70,173 @@ __device__ __forceinline__ void cmul_d(double2 &x, double ar, double ai) {
     x.x = fma(ar, x.x, p);
     x.y = fma(ar, x.y, q);
 }
-__device__ __forceinline__ MatD load_mat(const double *m) {
+__device__ __forceinline__ MatD load_mat_d(const double *m) {
     MatD M;
+    const double2 *v = reinterpret_cast<const double2 *>(m);
 #pragma unroll
-    for (int e = 0; e < 8; e++) M.m[e] = m[e];
+    for (int e = 0; e < 4; e++) {
+        const double2 x = v[e];
+        M.m[2 * e] = x.x;
+        M.m[2 * e + 1] = x.y;
+    }
     return M;
 }
 
-// Register-bit target RBIT: pairs (r, r | 2^RBIT). tok: the controls outside the register bits hold.
-template <int NV, int RBIT>
-__device__ __forceinline__ void reg_op_d(double2 (&A)[NV], const QsvOpD &op, bool tok) {
+#define QSV_PAIRS for (int r = 0; r < NV; r++) if (!(r & B))
+#define QSV_SEL if ((sel >> r) & 1u)
+template <int NV, int RBIT, bool R0>
+__device__ __forceinline__ void dense_op_d(double2 (&A)[NV], const MatD &M) {
     constexpr int B = 1 << RBIT;
-    const int cm = op.cm_reg;
-#define QSV_FOR_PAIRS for (int r = 0; r < NV; r++) if (!(r & B))
-    switch (op.variant) {
-        case QSV_V_UNI_DENSE: {
-            const MatD M = load_mat(op.m0);
-            if (op.r00) {
 #pragma unroll
-                QSV_FOR_PAIRS dense_r0_d(A[r], A[r | B], M);
-            } else {
-#pragma unroll
-                QSV_FOR_PAIRS dense_d(A[r], A[r | B], M);
-            }
-            break;
-        }
-        case QSV_V_UNI_SWAP:
-        case QSV_V_CTRL_SWAP:
-        case QSV_V_CTRL_SWAP_SEL:
-            // lanes of a warp whose controls do not hold sit the exchange out
-            if (tok) {
-#pragma unroll
-                QSV_FOR_PAIRS if ((r & cm) == cm) { const double2 t = A[r]; A[r] = A[r | B]; A[r | B] = t; }
-            }
-            break;
-        case QSV_V_CTRL_DENSE:
-        case QSV_V_CTRL_DENSE_SEL: {
-            const MatD M = load_mat(op.m1);
-            if (tok) {
-#pragma unroll
-                QSV_FOR_PAIRS if ((r & cm) == cm) dense_d(A[r], A[r | B], M);
-            }
-            break;
-        }
-        case QSV_V_MUX: {
-            const double *m0 = op.m0, *m1 = op.m1;
-#pragma unroll
-            QSV_FOR_PAIRS {
-                const bool s = tok && (r & cm) == cm;
-                MatD M;
-#pragma unroll
-                for (int e = 0; e < 8; e++) M.m[e] = s ? m1[e] : m0[e];
-                dense_d(A[r], A[r | B], M);
-            }
-            break;
-        }
-        default: break;
-    }
-#undef QSV_FOR_PAIRS
-}
-
-// Lane-bit target: each thread computes its own amplitudes as a*own + b*other, the other from the partner
-// lane, with (a, b) = (m00, m01) on the bit-0 side and (m11, m10) on the bit-1 side. Controls on register
-// bits are uniform (pairs outside them are left alone, no exchange); for controls elsewhere every lane
-// takes part in the exchange and keeps its amplitude where they do not hold.
-template <int NV>
-__device__ __forceinline__ void lane_op_d(double2 (&A)[NV], const QsvOpD &op, bool tok, int lanebit, int lane) {
-    const int xm = 1 << lanebit;
-    const bool mine = (lane >> lanebit) & 1;
-    const int cm = op.cm_reg;
-    auto partner = [&](const double2 &x) {
-        double2 o;
-        o.x = __shfl_xor_sync(0xffffffffu, x.x, xm);
-        o.y = __shfl_xor_sync(0xffffffffu, x.y, xm);
-        return o;
-    };
-    switch (op.variant) {
-        case QSV_V_UNI_SWAP:
-        case QSV_V_CTRL_SWAP:
-        case QSV_V_CTRL_SWAP_SEL:
-#pragma unroll
-            for (int r = 0; r < NV; r++)
-                if ((r & cm) == cm) {
-                    const double2 o = partner(A[r]);
-                    if (tok) A[r] = o;
-                }
-            break;
-        case QSV_V_UNI_DENSE:
-        case QSV_V_CTRL_DENSE:
-        case QSV_V_CTRL_DENSE_SEL: {
-            const double *m = op.kind == QSV_K_UNI ? op.m0 : op.m1;
-            const double ar = m[mine ? 6 : 0], ai = m[mine ? 7 : 1], br = m[mine ? 4 : 2], bi = m[mine ? 5 : 3];
-#pragma unroll
-            for (int r = 0; r < NV; r++)
-                if ((r & cm) == cm) {
-                    const double2 o = partner(A[r]);
-                    double2 y;
-                    lin_own_d(y.x, y.y, ar, ai, br, bi, A[r].x, A[r].y, o.x, o.y);
-                    if (tok) A[r] = y;
-                }
-            break;
-        }
-        case QSV_V_MUX: {
-#pragma unroll
-            for (int r = 0; r < NV; r++) {
-                const double *m = tok && (r & cm) == cm ? op.m1 : op.m0;
-                const double2 o = partner(A[r]);
-                double2 y;
-                lin_own_d(y.x, y.y, m[mine ? 6 : 0], m[mine ? 7 : 1], m[mine ? 4 : 2], m[mine ? 5 : 3], A[r].x, A[r].y,
-                          o.x, o.y);
-                A[r] = y;
-            }
-            break;
-        }
-        default: break;
+    QSV_PAIRS {
+        if (R0) dense_r0_d(A[r], A[r | B], M);
+        else dense_d(A[r], A[r | B], M);
     }
 }
-
-// Diagonal ops act on each amplitude alone, so their target may sit anywhere. With the target in the thread
-// (slots differ) or not (the thread's bit decides), diag(a, b) is a factor on the slots without and one on
-// the slots with it; controlled ops are diag(1, d): a factor on the slots with target and controls set.
+template <int NV, int RBIT>
+__device__ __forceinline__ void diag_op_d(double2 (&A)[NV], const MatD &M) {
+    constexpr int B = 1 << RBIT;
+#pragma unroll
+    QSV_PAIRS { cmul_d(A[r], M.m[0], M.m[1]); cmul_d(A[r | B], M.m[6], M.m[7]); }
+}
+template <int NV, int RBIT>
+__device__ __forceinline__ void cdense_op_d(double2 (&A)[NV], const MatD &M, uint32_t sel, bool tok) {
+    constexpr int B = 1 << RBIT;
+    if (tok) {
+#pragma unroll
+        QSV_PAIRS QSV_SEL dense_d(A[r], A[r | B], M);
+    }
+}
+template <int NV, int RBIT>
+__device__ __forceinline__ void swap_op_d(double2 (&A)[NV], uint32_t sel, bool tok) {
+    constexpr int B = 1 << RBIT;
+    if (tok) {
+#pragma unroll
+        QSV_PAIRS QSV_SEL { const double2 t = A[r]; A[r] = A[r | B]; A[r | B] = t; }
+    }
+}
+template <int NV, int RBIT>
+__device__ __forceinline__ void mux_op_d(double2 (&A)[NV], const MatD &M, const double *other, uint32_t sel, bool tok) {
+    constexpr int B = 1 << RBIT;
+    cdense_op_d<NV, RBIT>(A, M, sel, tok);
+    const MatD N = load_mat_d(other);
+    if (!tok) sel = 0;
+#pragma unroll
+    QSV_PAIRS if (!((sel >> r) & 1u)) dense_d(A[r], A[r | B], N);
+}
+// a factor on the slots whose index has every bit of RM
 template <int NV, int RM>
 __device__ __forceinline__ void phase_slots_d(double2 (&A)[NV], double ar, double ai) {
 #pragma unroll
     for (int r = 0; r < NV; r++)
         if ((r & RM) == RM) cmul_d(A[r], ar, ai);
 }
-template <int NV, int RB>
-__device__ __forceinline__ void diag_op_d(double2 (&A)[NV], const QsvOpD &op, uint32_t tb) {
-    const int slot = op.slot;
-    const bool reg = slot < QSV_SLOT_BASE, uni = op.kind == QSV_K_UNI;
-    int rm = op.cm_reg;
-    uint32_t thr = op.cm_thr;
-    if (reg) rm |= 1 << (slot - QSV_SLOT_REG0);
-    else thr |= 1u << op.tbit;
-    const bool on = (tb & thr) == thr;
-    const double *m = uni ? op.m0 : op.m1;
-    if (uni && op.cls == QSV_M_DIAG && (reg || !on)) {       // the amplitudes with the target bit clear
-        const double ar = m[0], ai = m[1];
-        switch (reg ? rm : 0) {
-            case 0: phase_slots_d<NV, 0>(A, ar, ai); break;
-            case 1:
-#pragma unroll
-                for (int r = 0; r < NV; r++) if (!(r & 1)) cmul_d(A[r], ar, ai);
-                break;
-            case 2:
-#pragma unroll
-                for (int r = 0; r < NV; r++) if (!(r & 2)) cmul_d(A[r], ar, ai);
-                break;
-            case 4:
-#pragma unroll
-                for (int r = 0; r < NV; r++) if (!(r & 4)) cmul_d(A[r], ar, ai);
-                break;
-            default:
-#pragma unroll
-                for (int r = 0; r < NV; r++) if (!(r & 8)) cmul_d(A[r], ar, ai);
-                break;
-        }
-    }
-    if (!on) return;
-    const double br = m[6], bi = m[7];
-    switch (rm) {
-        case 0: phase_slots_d<NV, 0>(A, br, bi); break;
-        case 1: phase_slots_d<NV, 1>(A, br, bi); break;
-        case 2: phase_slots_d<NV, 2>(A, br, bi); break;
-        case 3: phase_slots_d<NV, 3>(A, br, bi); break;
-        case 4: phase_slots_d<NV, 4>(A, br, bi); break;
-        case 5: phase_slots_d<NV, 5>(A, br, bi); break;
-        case 6: phase_slots_d<NV, 6>(A, br, bi); break;
-        case 8: phase_slots_d<NV, 8>(A, br, bi); break;
-        case 9: phase_slots_d<NV, 9>(A, br, bi); break;
-        case 10: phase_slots_d<NV, 10>(A, br, bi); break;
-        case 12: phase_slots_d<NV, 12>(A, br, bi); break;
-        default:
-#pragma unroll
-            for (int r = 7; r < NV; r++)
-                if ((r & rm) == rm) cmul_d(A[r], br, bi);
-            break;
-    }
+template <int NV>
+__device__ __forceinline__ void phase_op_d(double2 (&A)[NV], double ar, double ai, uint32_t rm) {
+    static_assert(NV == 8, "one case per mask");
+    if (rm == 0) phase_slots_d<NV, 0>(A, ar, ai);
+    else if (rm == 1) phase_slots_d<NV, 1>(A, ar, ai);
+    else if (rm == 2) phase_slots_d<NV, 2>(A, ar, ai);
+    else if (rm == 3) phase_slots_d<NV, 3>(A, ar, ai);
+    else if (rm == 4) phase_slots_d<NV, 4>(A, ar, ai);
+    else if (rm == 5) phase_slots_d<NV, 5>(A, ar, ai);
+    else if (rm == 6) phase_slots_d<NV, 6>(A, ar, ai);
+    else phase_slots_d<NV, 7>(A, ar, ai);
 }
 
-template <int NV, int RB>
-__device__ __forceinline__ void apply_op_d(const QsvOpD &op, double2 (&A)[NV], uint32_t tb, int lane) {
-    const int slot = op.slot, v = op.variant;
-    if (v == QSV_V_UNI_DIAG || v == QSV_V_CTRL_DIAG1 || v == QSV_V_CTRL_DIAG1_SEL) {
-        diag_op_d<NV, RB>(A, op, tb);
+// Lane-bit target: each thread computes its own amplitudes as a*own + b*other, the other from the partner lane, with
+// (a, b) = (m00, m01) on the bit-0 side and (m11, m10) on the bit-1 side. Controls on register bits are uniform
+// (slots outside them are left alone, no exchange); for controls elsewhere every lane takes part in the exchange
+// and keeps its amplitude where they do not hold.
+struct OwnD {
+    double ar, ai, br, bi;
+};
+__device__ __forceinline__ OwnD lane_own_d(const MatD &M, bool mine) {
+    return OwnD{mine ? M.m[6] : M.m[0], mine ? M.m[7] : M.m[1], mine ? M.m[4] : M.m[2], mine ? M.m[5] : M.m[3]};
+}
+__device__ __forceinline__ double2 shfl_d(const double2 &x, int xm) {
+    double2 o;
+    o.x = __shfl_xor_sync(0xffffffffu, x.x, xm);
+    o.y = __shfl_xor_sync(0xffffffffu, x.y, xm);
+    return o;
+}
+template <int NV>
+__device__ __forceinline__ void lane_dense_d(double2 (&A)[NV], const OwnD &M, int xm, uint32_t sel, bool keep) {
+#pragma unroll
+    for (int r = 0; r < NV; r++)
+        QSV_SEL {
+            const double2 o = shfl_d(A[r], xm);
+            double2 y;
+            lin_own_d(y.x, y.y, M.ar, M.ai, M.br, M.bi, A[r].x, A[r].y, o.x, o.y);
+            A[r].x = keep ? A[r].x : y.x;
+            A[r].y = keep ? A[r].y : y.y;
+        }
+}
+template <int NV>
+__device__ __forceinline__ void lane_op_d(double2 (&A)[NV], uint32_t path, uint32_t sel, uint32_t aux, const MatD &M,
+                                          const double *other, bool tok, int lane) {
+    const int xm = (int)(aux & 31u);
+    const bool mine = lane & xm;
+    if (path == QSV_P_LANE_SWAP) {
+#pragma unroll
+        for (int r = 0; r < NV; r++)
+            QSV_SEL {
+                const double2 o = shfl_d(A[r], xm);
+                A[r].x = tok ? o.x : A[r].x;
+                A[r].y = tok ? o.y : A[r].y;
+            }
         return;
     }
-    const bool tok = (tb & op.cm_thr) == op.cm_thr;
-    switch (slot) {
-        case QSV_SLOT_REG0 + 0: reg_op_d<NV, 0>(A, op, tok); break;
-        case QSV_SLOT_REG0 + 1: if constexpr (RB > 1) reg_op_d<NV, (RB > 1 ? 1 : 0)>(A, op, tok); break;
-        case QSV_SLOT_REG0 + 2: if constexpr (RB > 2) reg_op_d<NV, (RB > 2 ? 2 : 0)>(A, op, tok); break;
-        case QSV_SLOT_REG0 + 3: if constexpr (RB > 3) reg_op_d<NV, (RB > 3 ? 3 : 0)>(A, op, tok); break;
-        default: lane_op_d<NV>(A, op, tok, slot - QSV_SLOT_LANE0, lane); break;
+    const OwnD S = lane_own_d(M, mine);
+    if (path == QSV_P_LANE_DENSE) {
+        lane_dense_d<NV>(A, S, xm, 0xffffffffu, false);
+    } else if (path == QSV_P_LANE_CDENSE) {
+        lane_dense_d<NV>(A, S, xm, sel, !tok);
+    } else {                                     // QSV_P_LANE_MUX
+        const OwnD N = lane_own_d(load_mat_d(other), mine);
+        const OwnD T = {tok ? S.ar : N.ar, tok ? S.ai : N.ai, tok ? S.br : N.br, tok ? S.bi : N.bi};
+        lane_dense_d<NV>(A, T, xm, sel, false);
+        lane_dense_d<NV>(A, N, xm, ~sel, false);
     }
+}
+#undef QSV_PAIRS
+#undef QSV_SEL
+
+// The applied matrix is loaded before the path's branches so that both latencies overlap; vary: 0, unknown to be the
+// same in all lanes (lane_zero).
+template <int NV>
+__device__ __forceinline__ void apply_op_d(const uint4 &h, const QsvIOpD *op, double2 (&A)[NV], uint32_t tb, int lane,
+                                           uint32_t vary) {
+    const bool tok = (tb & h.x) == h.x;
+    const uint32_t path = h.y, sel = h.z, aux = h.w;
+    const MatD M = load_mat_d((op + vary)->a);
+#define QSV_BY_RBIT(G, CALL)                                        \
+    if (path == 4 * G) { constexpr int RBIT = 0; CALL; }            \
+    else if (path == 4 * G + 1) { constexpr int RBIT = 1; CALL; }   \
+    else { constexpr int RBIT = 2; CALL; }
+    if (path < 4 * (QSV_G_DENSE_R0 + 1)) {
+        QSV_BY_RBIT(QSV_G_DENSE_R0, (dense_op_d<NV, RBIT, true>(A, M)))
+    } else if (path < 4 * (QSV_G_DENSE + 1)) {
+        QSV_BY_RBIT(QSV_G_DENSE, (dense_op_d<NV, RBIT, false>(A, M)))
+    } else if (path == 4 * QSV_G_PHASE) {
+        if (tok) phase_op_d<NV>(A, M.m[6], M.m[7], aux);
+    } else if (path < 4 * (QSV_G_SWAP + 1)) {
+        QSV_BY_RBIT(QSV_G_SWAP, (swap_op_d<NV, RBIT>(A, sel, tok)))
+    } else if (path >= QSV_P_LANE_DENSE) {
+        if (path <= QSV_P_LANE_MUX) {
+            lane_op_d<NV>(A, path, sel, aux, M, op->b, tok, lane);
+        } else if (path == QSV_P_BASE_DIAG) {
+            const bool one = tb & aux;
+            phase_slots_d<NV, 0>(A, one ? M.m[6] : M.m[0], one ? M.m[7] : M.m[1]);
+        }
+    } else if (path < 4 * (QSV_G_DIAG + 1)) {
+        QSV_BY_RBIT(QSV_G_DIAG, (diag_op_d<NV, RBIT>(A, M)))
+    } else if (path < 4 * (QSV_G_CDENSE + 1)) {
+        QSV_BY_RBIT(QSV_G_CDENSE, (cdense_op_d<NV, RBIT>(A, M, sel, tok)))
+    } else {
+        QSV_BY_RBIT(QSV_G_MUX, (mux_op_d<NV, RBIT>(A, M, op->b, sel, tok)))
+    }
+#undef QSV_BY_RBIT
 }
 
 // the complex128 interpreter body: per phase, each thread loads its 2^RB amplitudes, applies the phase's
@@ -271,10 +245,29 @@ struct InterpBodyD {
     using Amp = double2;
     static constexpr int kHalfBits = 0;
     static constexpr bool kSmemOps = true;
+    using IOp = QsvIOpD;
+    // the expanded table follows the raw one (whose size keeps it on a 16-byte boundary)
+    static_assert(sizeof(QsvOpD) * QSV_MAX_SWEEP_OPS % 16 == 0, "expanded records are read as 16-byte vectors");
+    static __device__ __forceinline__ QsvIOpD *table(const QsvOpD *sops) {
+        return reinterpret_cast<QsvIOpD *>(const_cast<QsvOpD *>(sops) + QSV_MAX_SWEEP_OPS);
+    }
+    template <int NV>
+    static __device__ __forceinline__ void expand(const QsvOpD *sops, int nops, int tid, int nthreads) {
+        QsvIOpD *t = table(sops);
+        for (int i = tid; i < nops * 17; i += nthreads) {        // 16 coefficients and the header of each op
+            const int o = i / 17, e = i - o * 17;
+            const QsvOpD &op = sops[o];
+            if (e == 16) iop_header(op, NV, t[o]);
+            else if (e < 8) t[o].a[e] = op.kind == QSV_K_UNI ? op.m0[e] : op.m1[e];
+            else t[o].b[e - 8] = op.m0[e - 8];
+        }
+    }
     template <int NV, int RB, int WB>
     static __device__ __forceinline__ void tile(double2 *tile, const QsvSweepD &P, const QsvOpD *sops, int lane,
                                                 int warp, int bar) {
         constexpr int NC = 1 << (5 + WB);
+        const QsvIOpD *ops = table(sops);
+        const uint32_t vary = lane_zero();
         for (int ph = 0; ph < P.nphases; ph++) {
             if (ph > 0) named_bar_sync(bar, NC);
             const QsvPhase &Q = P.phases[ph];
@@ -304,7 +297,15 @@ struct InterpBodyD {
             double2 A[NV];
 #pragma unroll
             for (int r = 0; r < NV; r++) A[r] = tile[pos(r)];
-            for (int o = Q.op_begin; o < Q.op_end; o++) apply_op_d<NV, RB>(sops[o], A, tb, lane);
+            const int ob = Q.op_begin, oe = Q.op_end;
+            if (ob < oe) {
+                uint4 next = *reinterpret_cast<const uint4 *>(ops + ob);     // the next op's header, read ahead
+                for (int o = ob; o < oe; o++) {
+                    const uint4 h = next;
+                    if (o + 1 < oe) next = *reinterpret_cast<const uint4 *>(ops + o + 1);
+                    apply_op_d<NV>(h, ops + o, A, tb, lane, vary);
+                }
+            }
 #pragma unroll
             for (int r = 0; r < NV; r++) tile[pos(r)] = A[r];
         }
@@ -355,9 +356,9 @@ cudaError_t launch_sweep_c128(double2 *state, const QsvSweepD &sw, int nsm, cuda
     cudaError_t e = status_word_ptr(&status);
     if (e != cudaSuccess) return e;
     switch (sw.kw) {
-        case 12: return dev::launch_c128_t<12, 4, 3, 3>(state, sw, nsm, status, stream);
-        case 11: return dev::launch_c128_t<11, 4, 2, 3>(state, sw, nsm, status, stream);
-        case 10: return dev::launch_c128_t<10, 4, 1, 3>(state, sw, nsm, status, stream);
+        case 12: return dev::launch_c128_t<12, 3, 4, 3>(state, sw, nsm, status, stream);
+        case 11: return dev::launch_c128_t<11, 3, 3, 3>(state, sw, nsm, status, stream);
+        case 10: return dev::launch_c128_t<10, 3, 2, 3>(state, sw, nsm, status, stream);
         default: return cudaErrorInvalidValue;
     }
 }
