@@ -249,30 +249,52 @@ __device__ __forceinline__ void apply_op_p(const HdrP &h, const QsvIOp *op, p2 (
 #undef QSV_BY_RBIT
 }
 
+// A thread's place in a phase: tile index of its base, shared-memory positions of base and register bits (base and
+// register offsets are placed separately: swz128 is linear over XOR).
+template <int RB>
+struct PhaseAt {
+    uint32_t tb, base, rbit[RB];
+};
+template <int RB>
+__device__ __forceinline__ PhaseAt<RB> phase_at(const PhaseTab *t, int lane, int warp) {
+    PhaseAt<RB> p;
+    const uint32_t v = t->lane[lane] ^ t->warp[warp];
+    p.tb = v & 0xffffu;
+    p.base = v >> 16;
+    const uint4 r = *reinterpret_cast<const uint4 *>(t->rbit);
+    const uint32_t b[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int q = 0; q < RB; q++) p.rbit[q] = b[q];
+    return p;
+}
+// the same from a phase record, for a tile stored plainly (the batch kernel, whose phases are each run once)
+template <int RB, int WB, class PH>
+__device__ __forceinline__ PhaseAt<RB> phase_at(const PH &Q, int lane, int warp) {
+    PhaseAt<RB> p;
+    p.tb = ((uint32_t)(lane & 1) << Q.lane_lo[0]) | ((uint32_t)((lane >> 1) & 1) << Q.lane_lo[1]) |
+           ((uint32_t)((lane >> 2) & 1) << Q.lane_lo[2]) | ((uint32_t)((lane >> 3) & 1) << Q.lane_bits[0]) |
+           ((uint32_t)((lane >> 4) & 1) << Q.lane_bits[1]);
+#pragma unroll
+    for (int w = 0; w < WB; w++) p.tb |= (uint32_t)((warp >> w) & 1) << Q.warp_bits[w];
+    p.base = p.tb;
+#pragma unroll
+    for (int r = 0; r < RB; r++) p.rbit[r] = 1u << Q.reg_bits[r];
+    return p;
+}
+
 // One phase of a tile in shared memory: read the thread's 2^RB slots in the phase's layout, apply ops
-// [op_begin, op_end), write them back. PH is any phase record with reg_bits / lane_lo / lane_bits /
-// warp_bits; swz: the tile is stored swizzled. split_in / split_out: the slots hold (re0, re1, im0, im1),
-// the in-tile order between two phases (the two registers as they are), instead of the state's interleaved
-// order (first phase in, last phase out).
-template <int NV, int RB, int WB, class PH>
-__device__ __forceinline__ void run_phase(float2 *tile, const PH &Q, const QsvIOp *ops, int op_begin, int op_end,
-                                          int lane, int warp, uint32_t zero, bool swz = false,
-                                          bool split_in = false, bool split_out = false) {
-    uint32_t tb = ((uint32_t)(lane & 1) << Q.lane_lo[0]) | ((uint32_t)((lane >> 1) & 1) << Q.lane_lo[1]) |
-                  ((uint32_t)((lane >> 2) & 1) << Q.lane_lo[2]) | ((uint32_t)((lane >> 3) & 1) << Q.lane_bits[0]) |
-                  ((uint32_t)((lane >> 4) & 1) << Q.lane_bits[1]);
-#pragma unroll
-    for (int w = 0; w < WB; w++) tb |= (uint32_t)((warp >> w) & 1) << Q.warp_bits[w];
-    // shared-memory positions: base and register offsets swizzle separately (swz128 is linear over XOR)
-    const uint32_t base = swz ? swz128(tb) : tb;
-    uint32_t rbit[RB];
-#pragma unroll
-    for (int r = 0; r < RB; r++) rbit[r] = swz ? swz128(1u << Q.reg_bits[r]) : 1u << Q.reg_bits[r];
+// [op_begin, op_end), write them back. split_in / split_out: the slots hold (re0, re1, im0, im1), the in-tile order
+// between two phases (the two registers as they are), instead of the state's interleaved order (first phase in,
+// last phase out).
+template <int NV, int RB>
+__device__ __forceinline__ void run_phase(float2 *tile, const PhaseAt<RB> &at, const QsvIOp *ops, int op_begin,
+                                          int op_end, int lane, uint32_t zero, bool split_in, bool split_out) {
+    const uint32_t tb = at.tb;
     auto addr = [&](int r) -> uint32_t {
-        uint32_t o = base;
+        uint32_t o = at.base;
 #pragma unroll
         for (int q = 0; q < RB; q++)
-            if ((r >> q) & 1) o ^= rbit[q];
+            if ((r >> q) & 1) o ^= at.rbit[q];
         return o;
     };
     p2 R[NV], I[NV];

@@ -157,5 +157,29 @@ QSV_HD p2 iop_coef(const QsvOp &op, int e) {
     return pack2(-lo_m[i], -hi_m[i]);
 }
 
+// A phase's thread layout as the interpreters look it up: a thread's base is lane[lane] ^ warp[warp], the tile index in
+// the low half and its shared-memory position (swizzled or not) in the high half; rbit: positions of the register
+// bits. Spelled out from the phase record, a phase cost about a hundred instructions per tile and warp.
+struct alignas(16) PhaseTab {
+    uint32_t lane[32], warp[16], rbit[4];
+};
+// entry e (0..51) of a phase's table; pos(x): the position of tile index x (linear over XOR)
+template <class PH, class POS>
+QSV_HD uint32_t phase_entry(const PH &Q, int e, int rb, int wb, POS &&pos) {
+    uint32_t x = 0;
+    if (e < 32) {
+        for (int l = 0; l < 3; l++)
+            if ((e >> l) & 1) x |= 1u << Q.lane_lo[l];
+        for (int l = 0; l < 2; l++)
+            if ((e >> (3 + l)) & 1) x |= 1u << Q.lane_bits[l];
+    } else if (e < 48) {
+        for (int w = 0; w < wb; w++)
+            if (((e - 32) >> w) & 1) x |= 1u << Q.warp_bits[w];
+    } else {
+        return e - 48 < rb ? pos(1u << Q.reg_bits[e - 48]) : 0u;
+    }
+    return x | (pos(x) << 16);
+}
+
 }  // namespace dev
 }  // namespace qsv

@@ -44,6 +44,21 @@ struct InterpBody {
     static __device__ __forceinline__ QsvIOp *table(const QsvOp *sops) {
         return reinterpret_cast<QsvIOp *>(const_cast<QsvOp *>(sops) + QSV_MAX_SWEEP_OPS);
     }
+    // the phase tables take the raw ops' place
+    static __device__ __forceinline__ PhaseTab *phase_table(const QsvOp *sops) {
+        static_assert(sizeof(PhaseTab) * QSV_MAX_PHASES <= sizeof(QsvOp) * QSV_MAX_SWEEP_OPS, "phase tables fit");
+        return reinterpret_cast<PhaseTab *>(const_cast<QsvOp *>(sops));
+    }
+    template <int RB, int WB>
+    static __device__ __forceinline__ void expand_phases(const QsvOp *sops, const QsvSweep &P, int tid, int nthreads) {
+        const bool swz = P.swz != 0;
+        PhaseTab *pt = phase_table(sops);
+        for (int i = tid; i < P.nphases * 52; i += nthreads) {
+            const int ph = i / 52, e = i - ph * 52;
+            reinterpret_cast<uint32_t *>(pt + ph)[e] =
+                phase_entry(P.phases[ph], e, RB, WB, [&](uint32_t x) { return swz ? swz128(x) : x; });
+        }
+    }
     template <int NV>
     static __device__ __forceinline__ void expand(const QsvOp *sops, int nops, int tid, int nthreads) {
         QsvIOp *t = table(sops);
@@ -59,11 +74,12 @@ struct InterpBody {
                                                 int bar) {
         constexpr int NC = 1 << (5 + WB);
         const QsvIOp *iops = table(sops);
+        const PhaseTab *pt = phase_table(sops);
         for (int ph = 0; ph < P.nphases; ph++) {
             if (ph > 0) named_bar_sync(bar, NC);
             const QsvPhase &Q = P.phases[ph];
-            run_phase<NV, RB, WB>(tile, Q, iops, Q.op_begin, Q.op_end, lane, warp, P.zero, P.swz != 0, ph > 0,
-                                  ph + 1 < P.nphases);
+            run_phase<NV, RB>(tile, phase_at<RB>(pt + ph, lane, warp), iops, Q.op_begin, Q.op_end, lane, P.zero, ph > 0,
+                              ph + 1 < P.nphases);
         }
     }
 };

@@ -70,7 +70,8 @@ __device__ __forceinline__ void tma_store(const CUtensorMap *map, const int32_t 
 }
 
 // A body that reads its ops in another form names that record type IOp and fills the table, which follows the
-// raw one in shared memory, with expand(): the consumers do it while the first tiles are on their way.
+// raw one in shared memory, with expand(), then its phase tables over the raw ops, with expand_phases(): the consumers
+// do it while the first tiles are on their way.
 template <class T>
 struct VoidOf {
     typedef void type;
@@ -271,6 +272,8 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
     // ---------------------------------------------------------------- consumer warps
     if constexpr (ExpandedOps<Body>::value) {
         Body::template expand<NV>(sops, P.nops, tid, NC);
+        named_bar_sync(1, NC);
+        Body::template expand_phases<RB, WB>(sops, P, tid, NC);
         named_bar_sync(1, NC);
     }
     if constexpr (IL != 0) {

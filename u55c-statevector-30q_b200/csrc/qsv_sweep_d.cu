@@ -251,6 +251,22 @@ struct InterpBodyD {
     static __device__ __forceinline__ QsvIOpD *table(const QsvOpD *sops) {
         return reinterpret_cast<QsvIOpD *>(const_cast<QsvOpD *>(sops) + QSV_MAX_SWEEP_OPS);
     }
+    // the phase tables take the raw ops' place
+    static __device__ __forceinline__ PhaseTab *phase_table(const QsvOpD *sops) {
+        static_assert(sizeof(PhaseTab) * QSV_MAX_PHASES <= sizeof(QsvOpD) * QSV_MAX_SWEEP_OPS, "phase tables fit");
+        return reinterpret_cast<PhaseTab *>(const_cast<QsvOpD *>(sops));
+    }
+    template <int RB, int WB>
+    static __device__ __forceinline__ void expand_phases(const QsvOpD *sops, const QsvSweepD &P, int tid, int nthreads) {
+        // a swizzled tile holds amplitude x at x ^ ((x >> 3) & 7) (16-byte chunks, rows of 8)
+        const uint32_t sw = P.swz ? 7u : 0u;
+        PhaseTab *pt = phase_table(sops);
+        for (int i = tid; i < P.nphases * 52; i += nthreads) {
+            const int ph = i / 52, e = i - ph * 52;
+            reinterpret_cast<uint32_t *>(pt + ph)[e] =
+                phase_entry(P.phases[ph], e, RB, WB, [&](uint32_t x) { return x ^ ((x >> 3) & sw); });
+        }
+    }
     template <int NV>
     static __device__ __forceinline__ void expand(const QsvOpD *sops, int nops, int tid, int nthreads) {
         QsvIOpD *t = table(sops);
@@ -267,26 +283,15 @@ struct InterpBodyD {
                                                 int warp, int bar) {
         constexpr int NC = 1 << (5 + WB);
         const QsvIOpD *ops = table(sops);
+        const PhaseTab *pt = phase_table(sops);
         const uint32_t vary = lane_zero();
         for (int ph = 0; ph < P.nphases; ph++) {
             if (ph > 0) named_bar_sync(bar, NC);
             const QsvPhase &Q = P.phases[ph];
-            uint32_t tb = ((uint32_t)(lane & 1) << Q.lane_lo[0]) | ((uint32_t)((lane >> 1) & 1) << Q.lane_lo[1]) |
-                          ((uint32_t)((lane >> 2) & 1) << Q.lane_lo[2]) |
-                          ((uint32_t)((lane >> 3) & 1) << Q.lane_bits[0]) |
-                          ((uint32_t)((lane >> 4) & 1) << Q.lane_bits[1]);
-#pragma unroll
-            for (int w = 0; w < WB; w++) tb |= (uint32_t)((warp >> w) & 1) << Q.warp_bits[w];
-            // slot r at tile index tb | bits of r, a swizzled tile holding amplitude x at x ^ ((x >> 3) & 7)
-            // (16-byte chunks, rows of 8): linear over XOR, so base and register offsets swizzle separately
-            const uint32_t sw = P.swz ? 7u : 0u;
-            const uint32_t base = tb ^ ((tb >> 3) & sw);
-            uint32_t rbit[RB];
-#pragma unroll
-            for (int q = 0; q < RB; q++) {
-                const uint32_t x = 1u << Q.reg_bits[q];
-                rbit[q] = x ^ ((x >> 3) & sw);
-            }
+            const uint32_t v = pt[ph].lane[lane] ^ pt[ph].warp[warp];
+            const uint32_t tb = v & 0xffffu, base = v >> 16;
+            const uint4 rv = *reinterpret_cast<const uint4 *>(pt[ph].rbit);
+            const uint32_t rbit[4] = {rv.x, rv.y, rv.z, rv.w};
             auto pos = [&](int r) -> uint32_t {
                 uint32_t o = base;
 #pragma unroll
