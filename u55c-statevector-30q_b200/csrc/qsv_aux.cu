@@ -2,10 +2,10 @@
 //
 // remap: replaces the reference's exchange path -- sv_swap (kernels/sv/sv_swap.cpp:10-39) for
 // bank<->local transpositions and the host permutes of host/sv/runtime.py:261-268 -- with one in-HBM
-// sweep for an arbitrary bit permutation perm[new] = old (host/sv/model.py:74-78). Each CTA moves tiles
-// of 2^10 amplitudes that are contiguous in 32-amplitude runs on both sides: the tile holds source bits
-// 0..4 (coalesced reads) and the source bits that land on destination bits 0..4 (coalesced writes),
-// padded with the lowest remaining source bits; the transpose happens in shared memory.
+// sweep for an arbitrary bit permutation perm[new] = old (host/sv/model.py:74-78). Each CTA moves 32 KiB tiles
+// that are contiguous in 512-byte runs on both sides: the tile holds the lowest source bits (coalesced reads) and
+// the source bits that land on the lowest destination bits (coalesced writes), padded with the lowest remaining
+// source bits; the transpose happens in shared memory.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -17,116 +17,104 @@
 namespace qsv {
 namespace dev {
 
-#define REMAP_TB 11                 // tile bits: 2^11 amplitudes per tile (2^10 for a 10-qubit state)
-#define REMAP_RUN 5                 // contiguous run bits on each side (32 amplitudes per warp access)
+#define REMAP_TB 12                 // most tile bits
+#define REMAP_BANK_BITS 5           // a warp's shared-memory accesses vary five tile bits
 #define REMAP_THREADS 256
 
+// Everything linear in an index is given bit by bit: the bits of an index select terms that are combined with OR
+// (offsets) or XOR (shared-memory positions).
 struct RemapParams {
-    int n;
     int nfree;
-    uint8_t ubits[REMAP_TB];        // source bits of the tile, ascending (tile position bit i <-> ubits[i])
-    uint8_t fx[40];                 // free source bits, ascending
-    uint8_t fy[40];                 // destination position of free source bit fx[i]
-    uint8_t ypos[REMAP_TB];         // destination position of tile source bit ubits[i]
-    int8_t swz[REMAP_TB];           // shared-memory swizzle: tile bit b >= REMAP_RUN is XORed into low bit swz[b]
+    uint64_t roff[REMAP_TB];        // source offset of source-ordered tile position bit i
+    uint64_t woff[REMAP_TB];        // destination offset of destination-ordered tile position bit i
+    uint32_t spin[REMAP_TB];        // shared-memory position of source-ordered bit i
+    uint32_t spout[REMAP_TB];       // and of destination-ordered bit i
+    uint8_t fx[32];                 // source position of tile number bit i (free source bits, ascending)
+    uint8_t fy[32];                 // its destination position
 };
 
-// Bit permutation of the state, one HBM read and one write per amplitude. A tile is 2^11 amplitudes that
-// share the free bits (the source bits outside the tile); it holds source bits 0..4, so a warp's 32 reads
-// are contiguous, and the source bits that land on destination bits 0..4, so a warp's 32 writes are
-// contiguous. Shared memory holds the tile as 32-bit planes (W = sizeof(A) / 4 words per amplitude) at a
-// swizzled position: a warp's stores vary tile bits 0..4 and its loads vary the tile bits of destination
-// bits 0..4; the swizzle (host-chosen, linear) moves each such bit above bit 4 onto a low bit the other
-// four leave free, so both sides hit 32 distinct banks. Each thread's tile-invariant offsets are computed
-// once; the loads of the next tile are issued before the stores of the current one.
-// (three CTAs per SM: 80 registers, three tiles of loads in flight per SM plus each CTA's next tile)
+// Bit permutation of the state, one HBM read and one write per amplitude. A tile is 2^TB amplitudes that share the
+// free bits (the source bits outside the tile); it holds the lowest source bits, so that reads are contiguous in
+// runs of 512 bytes, and the source bits that land on the lowest destination bits, so that writes are too (2 x 6 bits
+// of complex64, 2 x 5 of complex128). Shared memory holds the tile as 32-bit planes (W = sizeof(A) / 4 words per
+// amplitude) at a swizzled position: a warp's stores vary tile bits 0..4 and its loads vary the tile bits of
+// destination bits 0..4; the swizzle (host-chosen, linear) moves each such bit above bit 4 onto a low bit the others
+// leave free, so both sides hit 32 distinct banks. The loads of the next tile are issued before the stores of the
+// current one. What bounds it: how much of HBM's rate scattered runs reach. With runs of 256 bytes (2^11-amplitude
+// tiles) and every thread's offsets in registers, a random permutation of 29 qubits took 1.63 ms (0.81 of the
+// measured copy rate), of 24 qubits 64 us; now 1.41 ms (0.93) and 48 us, complex128 at 28 qubits 1.70 -> 1.47 ms.
 template <class A, int TB>
 __global__ void __launch_bounds__(REMAP_THREADS, 3)
     remap_kernel(const A *__restrict__ src, A *__restrict__ dst, const __grid_constant__ RemapParams P) {
     constexpr int TS = 1 << TB;
-    constexpr int REMAP_EPT = TS / REMAP_THREADS;     // amplitudes per thread per tile
+    constexpr int EPT = TS / REMAP_THREADS;           // amplitudes per thread per tile: position bits 8..TB-1
     constexpr int W = sizeof(A) / 4;
     using Word = uint32_t;
-    __shared__ Word plane[W * TS];
-    const int t = threadIdx.x;
-    // destination enumeration: bit q of k walks the tile bit with the q-th smallest destination position
-    uint8_t order[TB];
-    {
-        bool used[TB] = {false};
-        for (int q = 0; q < TB; q++) {
-            int best = -1;
-            for (int i = 0; i < TB; i++)
-                if (!used[i] && (best < 0 || P.ypos[i] < P.ypos[best])) best = i;
-            used[best] = true;
-            order[q] = (uint8_t)best;
-        }
-    }
-    auto swz = [&](uint32_t j) -> uint32_t {
-        uint32_t m = 0;
-        for (int b = REMAP_RUN; b < TB; b++)
-            if (P.swz[b] >= 0 && ((j >> b) & 1)) m |= 1u << P.swz[b];
-        return j ^ m;
-    };
-    uint64_t ro[REMAP_EPT], wo[REMAP_EPT];
-    uint32_t sp_in[REMAP_EPT], sp_out[REMAP_EPT];
+    extern __shared__ Word plane[];                   // W * TS words
+    const int t = threadIdx.x, lane = t & 31;
+    uint64_t ro = 0, wo = 0;
+    uint32_t si = 0, so = 0;
 #pragma unroll
-    for (int e = 0; e < REMAP_EPT; e++) {
-        const uint32_t j = (uint32_t)(t + e * REMAP_THREADS);        // source-ordered tile position
+    for (int i = 0; i < 8; i++)
+        if ((t >> i) & 1) {
+            ro |= P.roff[i];
+            wo |= P.woff[i];
+            si ^= P.spin[i];
+            so ^= P.spout[i];
+        }
+    // the part of an offset that belongs to the thread's e-th amplitude (the same in all threads)
+    auto part64 = [](const uint64_t *off, int e) {
         uint64_t o = 0;
-        for (int i = 0; i < TB; i++)
-            if ((j >> i) & 1) o |= 1ull << P.ubits[i];
-        ro[e] = o;
-        sp_in[e] = swz(j);
-        const uint32_t k = j;                                         // destination-ordered enumeration
-        uint64_t w = 0;
-        uint32_t pos = 0;
-        for (int q = 0; q < TB; q++)
-            if ((k >> q) & 1) {
-                w |= 1ull << P.ypos[order[q]];
-                pos |= 1u << order[q];
-            }
-        wo[e] = w;
-        sp_out[e] = swz(pos);
-    }
-    auto bases = [&](int64_t T, uint64_t &xb, uint64_t &yb) {
-        xb = 0;
-        yb = 0;
-        for (uint64_t r = (uint64_t)T; r; r &= r - 1) {
-            const int i = __ffsll((long long)r) - 1;
-            xb |= 1ull << P.fx[i];
-            yb |= 1ull << P.fy[i];
-        }
-    };
-    const int64_t ntiles = 1ll << P.nfree;
-    int64_t T = blockIdx.x;
-    if (T >= ntiles) return;
-    A v[REMAP_EPT];
-    uint64_t xb, yb;
-    bases(T, xb, yb);
 #pragma unroll
-    for (int e = 0; e < REMAP_EPT; e++) v[e] = src[xb | ro[e]];
+        for (int k = 0; k < TB - 8; k++)
+            if ((e >> k) & 1) o |= off[8 + k];
+        return o;
+    };
+    auto part32 = [](const uint32_t *off, int e) {
+        uint32_t o = 0;
+#pragma unroll
+        for (int k = 0; k < TB - 8; k++)
+            if ((e >> k) & 1) o ^= off[8 + k];
+        return o;
+    };
+    // a tile's bases: lane i places bit i of the tile number
+    const uint64_t bx = lane < P.nfree ? 1ull << P.fx[lane] : 0, by = lane < P.nfree ? 1ull << P.fy[lane] : 0;
+    auto spread = [&](uint32_t T, uint64_t bit) {
+        const uint64_t x = (T >> lane) & 1u ? bit : 0;
+        return (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)x) |
+               ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32)) << 32);
+    };
+    const uint32_t ntiles = 1u << P.nfree;
+    uint32_t T = blockIdx.x;
+    if (T >= ntiles) return;
+    A v[EPT];
+    const A *s = src + (spread(T, bx) | ro);
+#pragma unroll
+    for (int e = 0; e < EPT; e++) v[e] = s[part64(P.roff, e)];
     while (true) {
 #pragma unroll
-        for (int e = 0; e < REMAP_EPT; e++) {
+        for (int e = 0; e < EPT; e++) {
             const Word *w = reinterpret_cast<const Word *>(&v[e]);
+            const uint32_t at = si ^ part32(P.spin, e);
 #pragma unroll
-            for (int p = 0; p < W; p++) plane[p * TS + sp_in[e]] = w[p];
+            for (int p = 0; p < W; p++) plane[p * TS + at] = w[p];
         }
         __syncthreads();
-        const uint64_t ycur = yb;
-        const int64_t Tn = T + gridDim.x;
+        A *d = dst + (spread(T, by) | wo);
+        const uint32_t Tn = T + gridDim.x;
         if (Tn < ntiles) {                      // next tile's loads in flight during this tile's stores
-            bases(Tn, xb, yb);
+            s = src + (spread(Tn, bx) | ro);
 #pragma unroll
-            for (int e = 0; e < REMAP_EPT; e++) v[e] = src[xb | ro[e]];
+            for (int e = 0; e < EPT; e++) v[e] = s[part64(P.roff, e)];
         }
 #pragma unroll
-        for (int e = 0; e < REMAP_EPT; e++) {
+        for (int e = 0; e < EPT; e++) {
             A a;
             Word *w = reinterpret_cast<Word *>(&a);
+            const uint32_t at = so ^ part32(P.spout, e);
 #pragma unroll
-            for (int p = 0; p < W; p++) w[p] = plane[p * TS + sp_out[e]];
-            dst[ycur | wo[e]] = a;
+            for (int p = 0; p < W; p++) w[p] = plane[p * TS + at];
+            d[part64(P.woff, e)] = a;
         }
         if (Tn >= ntiles) break;
         T = Tn;
@@ -521,27 +509,39 @@ __global__ void __launch_bounds__(32 * SAMPLE_WARPS)
 
 // ---------------------------------------------------------------- host launchers
 // dtype: 0 = complex64 (float2 amplitudes), 1 = complex128 (double2)
+template <class A, int TB>
+static cudaError_t launch_remap_t(const void *src, void *dst, const dev::RemapParams &P, int nsm, cudaStream_t stream) {
+    constexpr int smem = (int)(sizeof(A) << TB);
+    static_assert(smem <= 48 * 1024, "no opt-in needed");
+    const int64_t ntiles = 1ll << P.nfree;
+    int64_t grid = (int64_t)nsm * 3;
+    if (grid > ntiles) grid = ntiles;
+    dev::remap_kernel<A, TB><<<(unsigned)grid, REMAP_THREADS, smem, stream>>>((const A *)src, (A *)dst, P);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_remap(const void *src, void *dst, int n, const int32_t *perm, int dtype, int nsm,
                          cudaStream_t stream) {
     dev::RemapParams P;
     memset(&P, 0, sizeof(P));
-    P.n = n;
+    const int run = dtype ? 5 : 6;                         // 512-byte runs on both sides
+    const int most = 2 * run < REMAP_TB ? 11 : REMAP_TB;   // 32 KiB tiles
+    const int tbits = n < most ? n : most;
     int inv[64];
     for (int j = 0; j < n; j++) inv[perm[j]] = j;          // source bit perm[j] -> destination bit j
     bool in_tile[64] = {false};
     int cnt = 0;
-    for (int b = 0; b < REMAP_RUN; b++) { in_tile[b] = true; cnt++; }
-    for (int j = 0; j < REMAP_RUN; j++)
-        if (!in_tile[perm[j]]) { in_tile[perm[j]] = true; cnt++; }
-    const int tbits = n < REMAP_TB ? n : REMAP_TB;
+    // the lowest source and destination bits by turns (a small state's tile may not hold all of them)
+    for (int b = 0; b < run; b++) {
+        if (cnt < tbits && !in_tile[b]) { in_tile[b] = true; cnt++; }
+        if (cnt < tbits && !in_tile[perm[b]]) { in_tile[perm[b]] = true; cnt++; }
+    }
     for (int b = 0; b < n && cnt < tbits; b++)
         if (!in_tile[b]) { in_tile[b] = true; cnt++; }
-    int nu = 0, nf = 0;
+    int ubits[REMAP_TB], nu = 0, nf = 0;                   // tile position bit i <-> source bit ubits[i], ascending
     for (int b = 0; b < n; b++) {
         if (in_tile[b]) {
-            P.ubits[nu] = (uint8_t)b;
-            P.ypos[nu] = (uint8_t)inv[b];
-            nu++;
+            ubits[nu++] = b;
         } else {
             P.fx[nf] = (uint8_t)b;
             P.fy[nf] = (uint8_t)inv[b];
@@ -549,35 +549,43 @@ cudaError_t launch_remap(const void *src, void *dst, int n, const int32_t *perm,
         }
     }
     P.nfree = nf;
-    // swizzle: the tile bits carrying destination bits 0..4 vary across a warp's shared-memory loads; each of
-    // them above bit 4 is XORed onto a low bit (0..4) that none of the others occupies
-    for (int b = 0; b < REMAP_TB; b++) P.swz[b] = -1;
-    bool low_used[REMAP_RUN] = {false};
-    int hi[REMAP_RUN], nhi = 0;
-    for (int j = 0; j < REMAP_RUN; j++) {
-        int tb = -1;
+    // destination order: bit q walks the tile bit with the q-th smallest destination position
+    int order[REMAP_TB];
+    bool used[REMAP_TB] = {false};
+    for (int q = 0; q < nu; q++) {
+        int best = -1;
         for (int i = 0; i < nu; i++)
-            if (P.ubits[i] == perm[j]) tb = i;
-        if (tb < REMAP_RUN) low_used[tb] = true;
-        else hi[nhi++] = tb;
+            if (!used[i] && (best < 0 || inv[ubits[i]] < inv[ubits[best]])) best = i;
+        used[best] = true;
+        order[q] = best;
     }
-    for (int h = 0, slot = 0; h < nhi; h++) {
+    // swizzle: the tile bits that destination-order bits 0..4 walk vary across a warp's shared-memory loads; each of
+    // them above bit 4 is XORed onto a low bit (0..4) that none of the others occupies
+    int swz[REMAP_TB];
+    for (int b = 0; b < REMAP_TB; b++) swz[b] = -1;
+    bool low_used[REMAP_BANK_BITS] = {false};
+    for (int q = 0; q < REMAP_BANK_BITS; q++)
+        if (order[q] < REMAP_BANK_BITS) low_used[order[q]] = true;
+    for (int q = 0, slot = 0; q < REMAP_BANK_BITS; q++) {
+        if (order[q] < REMAP_BANK_BITS) continue;
         while (low_used[slot]) slot++;
-        P.swz[hi[h]] = (int8_t)slot;
+        swz[order[q]] = slot;
         low_used[slot] = true;
     }
-    const int64_t ntiles = 1ll << nf;
-    int64_t grid = (int64_t)nsm * 3;
-    if (grid > ntiles) grid = ntiles;
-    const unsigned g = (unsigned)grid;
-    if (tbits == REMAP_TB) {
-        if (dtype) dev::remap_kernel<double2, REMAP_TB><<<g, REMAP_THREADS, 0, stream>>>((const double2 *)src, (double2 *)dst, P);
-        else dev::remap_kernel<float2, REMAP_TB><<<g, REMAP_THREADS, 0, stream>>>((const float2 *)src, (float2 *)dst, P);
-    } else {                                  // a 10-qubit state is one tile of 2^10
-        if (dtype) dev::remap_kernel<double2, 10><<<g, REMAP_THREADS, 0, stream>>>((const double2 *)src, (double2 *)dst, P);
-        else dev::remap_kernel<float2, 10><<<g, REMAP_THREADS, 0, stream>>>((const float2 *)src, (float2 *)dst, P);
+    auto place = [&](int b) { return (1u << b) ^ (swz[b] >= 0 ? 1u << swz[b] : 0u); };
+    for (int i = 0; i < nu; i++) {
+        P.roff[i] = 1ull << ubits[i];
+        P.woff[i] = 1ull << inv[ubits[order[i]]];
+        P.spin[i] = place(i);
+        P.spout[i] = place(order[i]);
     }
-    return cudaGetLastError();
+    if (dtype) {
+        if (tbits == 11) return launch_remap_t<double2, 11>(src, dst, P, nsm, stream);
+        return launch_remap_t<double2, 10>(src, dst, P, nsm, stream);
+    }
+    if (tbits == 12) return launch_remap_t<float2, 12>(src, dst, P, nsm, stream);
+    if (tbits == 11) return launch_remap_t<float2, 11>(src, dst, P, nsm, stream);
+    return launch_remap_t<float2, 10>(src, dst, P, nsm, stream);
 }
 
 cudaError_t launch_copy_probe(void *dst, const void *src, size_t bytes, int nsm, cudaStream_t stream) {
