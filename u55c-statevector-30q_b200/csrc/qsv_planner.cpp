@@ -223,7 +223,7 @@ static int tma_dims(const SW &sw, TmaDims &D, bool swz = false) {
 // Ops [b, e) in tile coordinates of a window (tile_of[q] = tile bit of physical qubit q) with their matrix
 // classes, kinds and code variants (independent of the thread layout).
 template <class OpT>
-static void classify_ops(const std::vector<PhysOp> &ops, size_t b, size_t e, const int *tile_of, int n,
+static void classify_ops(const std::vector<PhysOp> &ops, size_t b, size_t e, const int *tile_of,
                          std::vector<OpT> &out) {
     constexpr bool C128 = std::is_same<OpT, QsvOpD>::value;
     out.assign(e - b, OpT());
@@ -234,8 +234,7 @@ static void classify_ops(const std::vector<PhysOp> &ops, size_t b, size_t e, con
         set_mats(o, p);
         o.tbit = (uint8_t)tile_of[p.t];
         o.cmask = 0;
-        for (int q = 0; q < n; q++)
-            if ((p.cmask >> q) & 1) o.cmask |= 1u << tile_of[q];
+        for (uint64_t c = p.cmask; c; c &= c - 1) o.cmask |= 1u << tile_of[__builtin_ctzll(c)];
         o.cls0 = classify(o.m0);
         o.cls1 = classify(o.m1);
         // identical matrices, or a control on the target bit (i0 never has it set): M1 is never
@@ -265,7 +264,14 @@ static void classify_ops(const std::vector<PhysOp> &ops, size_t b, size_t e, con
     }
 }
 
-// The phases of classified ops, greedy in op order, and each op's slot and layout-dependent fields. Plain
+// diagonal ops act on each amplitude alone
+template <class OpT>
+static bool elementwise_op(const OpT &o) {
+    return o.variant == QSV_V_SKIP || o.variant == QSV_V_UNI_DIAG || o.variant == QSV_V_CTRL_DIAG1 ||
+           o.variant == QSV_V_CTRL_DIAG1_SEL ||
+           (o.variant == QSV_V_MUX && o.kind == QSV_K_CTRL && o.cls1 == QSV_M_DIAG1);
+}
+// The phases of classified ops, greedy in op order, and how many of the ops are warp-shuffle ops in them. Plain
 // layout: tile bits above the fixed lane bits (>= 4 for complex64, whose tile bit 0 is the packed half of a
 // float4 and bits 1-3 are lanes; >= 3 for complex128, bits 0-2 lanes) that are targets need a register or
 // lane slot. swz: the swizzled layout, in which lane bit l (0-2) sits on tile bit F+l or F+3+l (F = 1 for
@@ -274,25 +280,26 @@ static void classify_ops(const std::vector<PhysOp> &ops, size_t b, size_t e, con
 // act on each amplitude alone, need no slot (a target left on a warp bit gets QSV_SLOT_BASE), and complex64 ops
 // are laid out for the interpreter (layout_interp).
 template <class OpT>
-static bool elementwise_op(const OpT &o) {
-    return o.variant == QSV_V_SKIP || o.variant == QSV_V_UNI_DIAG || o.variant == QSV_V_CTRL_DIAG1 ||
-           o.variant == QSV_V_CTRL_DIAG1_SEL ||
-           (o.variant == QSV_V_MUX && o.kind == QSV_K_CTRL && o.cls1 == QSV_M_DIAG1);
+static int layout_of(int kw, bool free_diag, int *rb, int *wb, std::string &err) {
+    // (the callers plan for the interpreter exactly when diagonal ops need no slot)
+    if (std::is_same<OpT, QsvOpD>::value ? layout_for_kw_c128(kw, rb, wb)
+                                         : free_diag ? layout_interp(kw, rb, wb) : layout_for_kw(kw, rb, wb)) {
+        err = "unsupported window size";
+        return QSV_ERR_UNSUPPORTED;
+    }
+    return QSV_OK;
 }
 template <class OpT>
-static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &phases, std::string &err,
-                       bool swz, int lane_cap, bool free_diag = false) {
-    // (the callers plan for the interpreter exactly when diagonal ops need no slot)
+static int layout_phases(const std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &phases, int *lane_ops,
+                         std::string &err, bool swz, int lane_cap, bool free_diag) {
     constexpr bool C128 = std::is_same<OpT, QsvOpD>::value;
     constexpr int FIXED_LO = C128 ? 0 : 1;       // first tile bit on lane bits 0-2
     constexpr int FREE_LO = FIXED_LO + 3;        // tile bits from here on need a slot when targeted
     int rb, wb;
-    if (C128 ? layout_for_kw_c128(kw, &rb, &wb)
-             : free_diag ? layout_interp(kw, &rb, &wb) : layout_for_kw(kw, &rb, &wb)) {
-        err = "unsupported window size";
-        return QSV_ERR_UNSUPPORTED;
-    }
+    const int lrc = layout_of<OpT>(kw, free_diag, &rb, &wb, err);
+    if (lrc) return lrc;
     phases.clear();
+    *lane_ops = 0;
     const size_t nops = out.size();
     // swizzled layout: tile bits FIXED_LO + l and FIXED_LO + 3 + l pair up on lane bit l
     auto pair_of = [&](int t) { return (swz && t >= FIXED_LO && t < FIXED_LO + 6) ? (t - FIXED_LO) % 3 : -1; };
@@ -308,8 +315,11 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
     // rb + g_phase_lanes over tile bits >= FREE_LO, whose lane bits 0-2 are fixed.
     auto assign = [&](const int *used, const int *cnt, int nu, Assign &A) -> bool {
         int order[QSV_KW_MAX];
-        for (int u = 0; u < nu; u++) order[u] = u;
-        std::stable_sort(order, order + nu, [&](int x, int y) { return cnt[x] > cnt[y]; });
+        for (int u = 0; u < nu; u++) {                     // by use, ties in order of appearance
+            int at = u;
+            for (; at > 0 && cnt[order[at - 1]] < cnt[u]; at--) order[at] = order[at - 1];
+            order[at] = u;
+        }
         A.nr = 0;
         A.nf = 0;
         A.pl[0] = A.pl[1] = A.pl[2] = -1;
@@ -385,6 +395,27 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
         ph.lane_bits[1] = (uint8_t)lanes[1];
         ph.op_begin = (int32_t)i;
         ph.op_end = (int32_t)j;
+        uint32_t lanemask = (1u << ph.lane_bits[0]) | (1u << ph.lane_bits[1]);
+        for (int l = 0; l < 3; l++) lanemask |= 1u << ph.lane_lo[l];
+        for (size_t o = i; o < j; o++)
+            *lane_ops += (lanemask >> out[o].tbit & 1u) && (C128 || out[o].tbit) && out[o].variant != QSV_V_SKIP &&
+                         !(free_diag && elementwise_op(out[o]));
+        phases.push_back(ph);
+        i = j;
+    }
+    return QSV_OK;
+}
+
+// Each op's slot and layout-dependent fields in its phase.
+template <class OpT>
+static int place_ops(std::vector<OpT> &out, int kw, const std::vector<QsvPhaseX> &phases, bool free_diag,
+                     std::string &err) {
+    constexpr bool C128 = std::is_same<OpT, QsvOpD>::value;
+    int rb, wb;
+    const int lrc = layout_of<OpT>(kw, free_diag, &rb, &wb, err);
+    if (lrc) return lrc;
+    for (const QsvPhaseX &ph : phases) {
+        const size_t i = (size_t)ph.op_begin, j = (size_t)ph.op_end;
         uint32_t regmask = 0;
         for (int r = 0; r < rb; r++) regmask |= 1u << ph.reg_bits[r];
         uint32_t lanemask = (1u << ph.lane_bits[0]) | (1u << ph.lane_bits[1]);
@@ -418,8 +449,6 @@ static int plan_phases(std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &ph
                 else if (op.variant == QSV_V_CTRL_SWAP) op.variant = QSV_V_CTRL_SWAP_SEL;
             }
         }
-        phases.push_back(ph);
-        i = j;
     }
     return QSV_OK;
 }
@@ -428,13 +457,15 @@ template <class OpT>
 static int plan_window(const std::vector<PhysOp> &ops, size_t b, size_t e, const int *tile_of, int n, int kw,
                        std::vector<OpT> &out, std::vector<QsvPhaseX> &phases, std::string &err, bool swz = false,
                        int lane_cap = 8, bool free_diag = false) {
-    classify_ops<OpT>(ops, b, e, tile_of, n, out);
-    return plan_phases<OpT>(out, kw, phases, err, swz, lane_cap, free_diag);
+    classify_ops<OpT>(ops, b, e, tile_of, out);
+    int lane_ops = 0;
+    const int rc = layout_phases<OpT>(out, kw, phases, &lane_ops, err, swz, lane_cap, free_diag);
+    return rc ? rc : place_ops<OpT>(out, kw, phases, free_diag, err);
 }
 
 // The phases of a sweep's classified ops (window and n set), in the plain layout or a swizzled one.
 template <class OpT>
-static int choose_layout(QsvSweepT<OpT> &sw, const std::vector<OpT> &base, bool free_diag, std::string &err) {
+static int choose_layout(QsvSweepT<OpT> &sw, std::vector<OpT> &ops, bool free_diag, std::string &err) {
     const int kw = sw.kw;
     auto set_dims = [&](const TmaDims &D) {
         sw.tma_rank = (uint8_t)D.rank;
@@ -445,43 +476,35 @@ static int choose_layout(QsvSweepT<OpT> &sw, const std::vector<OpT> &base, bool 
     sw.swz = 0;
     sw.tma_rank = sw.tma_xbits = 0;
     if (tma_dims(sw, dims)) set_dims(dims);
-    std::vector<OpT> vops = base;
-    std::vector<QsvPhaseX> vph;
-    int rc = plan_phases<OpT>(vops, kw, vph, err, false, 8, free_diag);
+    std::vector<QsvPhaseX> vph, sph;
+    int lane = 0;
+    int rc = layout_phases<OpT>(ops, kw, vph, &lane, err, false, 8, free_diag);
     if (rc) return rc;
-    auto lane_ops = [&](const std::vector<OpT> &o) {
-        int lane = 0;
-        for (const OpT &x : o)
-            lane += x.slot >= QSV_SLOT_LANE0 && x.variant != QSV_V_SKIP && !(free_diag && elementwise_op(x));
-        return lane;
-    };
     // the swizzled layout where it costs less: cost = lane ops + 2 per phase change (a shared-memory round
     // trip moves as many bytes through the shared-memory pipe as two shuffle ops); ties keep the plain one
-    if (swizzle_enabled() && (lane_ops(vops) > 0 || (free_diag && vph.size() > 1))) {
-        const int r = tma_dims(sw, dims, true);
+    if (swizzle_enabled() && (lane > 0 || (free_diag && vph.size() > 1)) && tma_dims(sw, dims, true)) {
         // QSV_PHASE_COST overrides the weight of a phase change (tuning studies)
         static const int phase_cost = [] {
             const char *e = std::getenv("QSV_PHASE_COST");
             return e ? std::atoi(e) : 2;
         }();
-        auto cost = [&](const std::vector<OpT> &o, const std::vector<QsvPhaseX> &p) {
-            return lane_ops(o) + phase_cost * ((int)p.size() - 1);
-        };
+        int best = lane + phase_cost * ((int)vph.size() - 1);
         // phases with fewer shuffle ops but more round trips, or the reverse: try lane-op budgets per phase
         for (int cap : {0, 1, 2, 8}) {
-            if (!r) break;
-            std::vector<OpT> sops = base;
-            std::vector<QsvPhaseX> sph;
             std::string serr;
-            if (plan_phases<OpT>(sops, kw, sph, serr, true, cap, free_diag) == QSV_OK &&
-                sph.size() <= QSV_MAX_PHASES && cost(sops, sph) < cost(vops, vph)) {
-                vops.swap(sops);
+            if (layout_phases<OpT>(ops, kw, sph, &lane, serr, true, cap, free_diag) != QSV_OK) continue;
+            const int c = lane + phase_cost * ((int)sph.size() - 1);
+            if (sph.size() <= QSV_MAX_PHASES && c < best) {
                 vph.swap(sph);
+                best = c;
                 sw.swz = 1;
                 set_dims(dims);
             }
         }
     }
+    rc = place_ops<OpT>(ops, kw, vph, free_diag, err);
+    if (rc) return rc;
+    const std::vector<OpT> &vops = ops;
     if (vops.size() > QSV_MAX_SWEEP_OPS || vph.size() > QSV_MAX_PHASES) { err = "sweep too large"; return QSV_ERR_UNSUPPORTED; }
     sw.nops = (int)vops.size();
     sw.nphases = (int)vph.size();
@@ -523,7 +546,7 @@ static int fill_sweep(const std::vector<PhysOp> &ops, size_t b, size_t e, uint64
     sw.nh = nh;
     sw.ntiles = 1ll << (n - kw);
     std::vector<OpT> base;
-    classify_ops<OpT>(ops, b, e, tile_of, n, base);
+    classify_ops<OpT>(ops, b, e, tile_of, base);
     // complex128 sweeps only ever run on their interpreter
     return choose_layout<OpT>(sw, base, C128 || interp, err);
 }
@@ -552,6 +575,9 @@ int build_sweeps(const std::vector<PhysPass> &passes, int n, int kw, int lo_merg
                  std::vector<QsvSweepT<OpT>> &out, std::string &err, bool interp) {
     out.clear();
     std::vector<PhysOp> ops;
+    size_t total = 0;
+    for (const PhysPass &p : passes) total += p.ops.size();
+    ops.reserve(total);
     uint64_t cur = 0;
     size_t begin = 0;
     auto flush = [&]() -> int {
