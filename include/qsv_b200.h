@@ -195,15 +195,15 @@ QSV_API int qsv_set_phase_lanes(int k);
  * 2 = automatic (default): a structure is compiled in background threads once its launches have swept
  * 2^31 amplitudes in total (two sweeps of a 30-qubit state, 512 of a 22-qubit one; at most 64 compilations
  * wait at a time), and used from the first launch after its kernel is ready; until then the sweep runs its
- * coarse structure's kernel, compiled once the sweeps sharing it have swept 2^30 amplitudes, or (13-qubit
- * windows) the group-type library, or the interpreter; 3 = eager with coarse structures only; 4 = the
- * group-type library only (qsv_jit_prepare builds it, blocking, to cover a segment's 13-qubit sweeps).
+ * coarse structure's kernel, compiled once the sweeps sharing it have swept 2^30 amplitudes, or the
+ * interpreter; 3 = eager with coarse structures only; 4 = the group-type library where it covers a sweep
+ * (qsv_jit_prepare builds it, blocking, to cover a segment's 13-qubit sweeps), else the interpreter.
  * The group-type library is a set of up to 8 kernels, each with straight-line code for 32 op sequences of
  * one group of the streaming form (per op: slot among the group's three item bits, code variant, kind,
  * matrix classes): the 16 that have swept the most amplitudes and a band of 16 more, with item bits,
- * control masks and matrices read at run time. A sweep whose exact and coarse structures never repeat
- * takes the kernel that covers most of its ops, once 3/4 of them fall in its cases; the set is rebuilt in
- * the background after groups outside it have swept 2^31 amplitudes.
+ * control masks and matrices read at run time. In mode 4 a 13-qubit sweep takes the kernel that covers most
+ * of its ops, once 3/4 of them fall in its cases; the set is rebuilt in the background after groups outside
+ * it have swept 2^31 amplitudes. (The automatic mode does not use it: the interpreter is as fast.)
  * Switching to mode 0 drops waiting compilations and waits for running ones. Returns the previous mode.
  * Process-wide. */
 QSV_API int qsv_set_jit(int mode);
@@ -216,8 +216,7 @@ QSV_API int qsv_jit_prepare(const int32_t *seg, size_t nwords, int n);
 
 /* Build (blocking, host work only) the group-type library (qsv_set_jit) from the 13-qubit sweeps of count
  * programs (segment i: segs[i], nwords[i] words, for an ns[i]-qubit state): their group types' swept
- * amplitudes are recorded and the libraries take the most swept types seen so far (up to 144). A batch or a service
- * calls it once before its timed or latency-bound work. Returns the number of types in the library, or a
+ * amplitudes are recorded and the libraries take the most swept types seen so far (up to 144), for mode 4. Returns the number of types in the library, or a
  * negative error code (malformed segment; QSV_ERR_CUDA if the library does not compile). */
 QSV_API int qsv_jit_prepare_library(const int32_t *const *segs, const size_t *nwords, const int *ns, int count);
 

@@ -401,10 +401,9 @@ def inject_skip_load(count=1):
 def set_jit(mode):
     """Specialised sweep kernels: "off" (interpreter only), "eager" (compile each new sweep structure before
     its first launch), "auto" (default: compile in the background once a structure's launches have swept
-    2^31 amplitudes; meanwhile use the kernel of its coarse structure or, on 13-qubit windows, the group-type
-    library when ready), "coarse" (eager, coarse structures only) or "library" (the group-type library only;
-    jit_prepare builds it for a segment, jit_prepare_library for many programs). Values are identical in
-    every mode. Returns the previous mode's name."""
+    2^31 amplitudes; meanwhile use the kernel of its coarse structure when ready, or the interpreter), "coarse"
+    (eager, coarse structures only) or "library" (the group-type library where it covers a sweep; jit_prepare
+    builds it for a segment, jit_prepare_library for many programs). Values are identical in every mode. Returns the previous mode's name."""
     rc = load().qsv_set_jit(JIT_MODES[mode] if isinstance(mode, str) else int(mode))
     if rc < 0:
         _check(rc)
