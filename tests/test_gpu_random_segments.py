@@ -6,7 +6,7 @@ import sys
 import numpy as np
 import pytest
 
-from qsv_b200 import compile_circuit, engine
+from qsv_b200 import compile_circuit, engine, isa
 from qsv_b200.generators import random_layer
 from oracle import oracle as orc
 
@@ -63,4 +63,37 @@ def test_random_segments_specialised_exact(shape, mode):
             x = orc.run_segment(x.copy(), seg)
             assert np.array_equal(t.cpu().numpy(), x)
     finally:
+        engine.set_jit(old)
+
+
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+@pytest.mark.parametrize("lanes", [0, 1, 2])
+@pytest.mark.parametrize("n", [11, 12, 13])
+def test_most_phases(n, lanes, dtype):
+    """96 ops whose targets never repeat within a phase: as many phases as a sweep can need, whatever the knob."""
+    torch = pytest.importorskip("torch")
+    k = min(n, 12)
+    seg = random_segment(n, k, 2, 48, n, dtype).copy()
+    words = isa.OP_WORDS_C128 if dtype == "c128" else isa.OP_WORDS
+    at = isa.HDR_WORDS
+    for p in range(2):
+        seg[at:at + 8] = [0, 0, 0, 48, 0, 0, 0, 0]
+        at += isa.PASS_WORDS
+        for o in range(48):
+            rec = seg[at:at + words]
+            mats = rec[8:].view(np.float64 if dtype == "c128" else np.float32)
+            mats[:8] = mats[8:] = [0.6, 0.1, 0.3, -0.5, -0.3, -0.5, 0.6, -0.1]        # dense: needs a slot
+            rec[1], rec[2] = 3 + (5 * o) % (k - 3), 0
+            at += words
+    x = random_state(n, n, dtype)
+    old = engine.set_jit("off")
+    engine.set_phase_lanes(lanes)
+    try:
+        t = torch.from_numpy(x.copy()).cuda()
+        engine.run_segment(t, seg)
+        torch.cuda.synchronize()
+        assert engine.device_status() == 0
+        assert np.array_equal(t.cpu().numpy(), orc.run_segment(x.copy(), seg))
+    finally:
+        engine.set_phase_lanes(1)
         engine.set_jit(old)

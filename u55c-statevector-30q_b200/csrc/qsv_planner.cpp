@@ -291,7 +291,7 @@ static int layout_of(int kw, bool free_diag, int *rb, int *wb, std::string &err)
 }
 template <class OpT>
 static int layout_phases(const std::vector<OpT> &out, int kw, std::vector<QsvPhaseX> &phases, int *lane_ops,
-                         std::string &err, bool swz, int lane_cap, bool free_diag) {
+                         std::string &err, bool swz, int lane_cap, bool free_diag, int min_lanes = 0) {
     constexpr bool C128 = std::is_same<OpT, QsvOpD>::value;
     constexpr int FIXED_LO = C128 ? 0 : 1;       // first tile bit on lane bits 0-2
     constexpr int FREE_LO = FIXED_LO + 3;        // tile bits from here on need a slot when targeted
@@ -300,6 +300,7 @@ static int layout_phases(const std::vector<OpT> &out, int kw, std::vector<QsvPha
     if (lrc) return lrc;
     phases.clear();
     *lane_ops = 0;
+    const int max_fl = std::max(g_phase_lanes, min_lanes);      // targets on lane bits 3-4
     const size_t nops = out.size();
     // swizzled layout: tile bits FIXED_LO + l and FIXED_LO + 3 + l pair up on lane bit l
     auto pair_of = [&](int t) { return (swz && t >= FIXED_LO && t < FIXED_LO + 6) ? (t - FIXED_LO) % 3 : -1; };
@@ -332,7 +333,7 @@ static int layout_phases(const std::vector<OpT> &out, int kw, std::vector<QsvPha
             const int nlane = A.nf + (A.pl[0] >= 0) + (A.pl[1] >= 0) + (A.pl[2] >= 0);
             if (A.nr < rb && !partner_reg) A.regs[A.nr++] = t;
             else if (l >= 0 && A.pl[l] < 0 && nlane < lane_cap) A.pl[l] = t;
-            else if (A.nf < g_phase_lanes && nlane < lane_cap) A.fl[A.nf++] = t;
+            else if (A.nf < max_fl && nlane < lane_cap) A.fl[A.nf++] = t;
             else return false;
         }
         return true;
@@ -480,6 +481,13 @@ static int choose_layout(QsvSweepT<OpT> &sw, std::vector<OpT> &ops, bool free_di
     int lane = 0;
     int rc = layout_phases<OpT>(ops, kw, vph, &lane, err, false, 8, free_diag);
     if (rc) return rc;
+    if (vph.size() > QSV_MAX_PHASES) {
+        // more phases than a sweep holds: with both free lane bits for targets a phase takes at least four of them
+        // (two register bits or more), so QSV_MAX_SWEEP_OPS ops fit
+        static_assert(QSV_MAX_SWEEP_OPS <= 4 * QSV_MAX_PHASES, "four ops or more per phase");
+        rc = layout_phases<OpT>(ops, kw, vph, &lane, err, false, 8, free_diag, 2);
+        if (rc) return rc;
+    }
     // the swizzled layout where it costs less: cost = lane ops + 2 per phase change (a shared-memory round
     // trip moves as many bytes through the shared-memory pipe as two shuffle ops); ties keep the plain one
     if (swizzle_enabled() && (lane > 0 || (free_diag && vph.size() > 1)) && tma_dims(sw, dims, true)) {
