@@ -1,10 +1,11 @@
-// qsv_ops.cuh -- in-register application of MUX2 ops for the tile kernels (sweep and batch).
+// qsv_ops.cuh -- in-register application of MUX2 ops for the streaming kernels, and pair arithmetic with the matrix
+// class fixed for the specialised ones. (The phase interpreter and the specialised kernels' packed arithmetic:
+// qsv_packed.cuh.)
 //
-// A consumer thread keeps 2^RB float4 of its tile (the two halves of each float4 = tile bit 0) repacked
-// as float2 (re, re) / (im, im) pairs, so one packed FP32x2 FMA updates two amplitude pairs. Ops on tile
-// bit 0 pair the halves of a float4 (scalar arithmetic), ops on register bits pair two float4, ops on lane
-// bits exchange with the partner lane by warp shuffles. The arithmetic is the canonical fused-multiply-add
-// chain of qsv_device.cuh for every variant (the specialised variants only skip exact-zero terms).
+// An item's float4 (the two halves of each = tile bit 0) are kept repacked as float2 (re, re) / (im, im) pairs, so one
+// packed FP32x2 FMA updates two amplitude pairs. Ops on tile bit 0 pair the halves of a float4 (scalar arithmetic),
+// ops on item bits pair two float4. The arithmetic is the canonical fused-multiply-add chain of qsv_device.cuh for
+// every variant (the specialised variants only skip exact-zero terms).
 #pragma once
 #include "qsv_device.cuh"
 
@@ -217,69 +218,7 @@ __device__ __forceinline__ void comp_op(float2 (&R)[NV], float2 (&I)[NV], const 
     }
 }
 
-// lane-bit target: exchange with the partner lane; each thread computes its own amplitude as
-// a * own + b * other with (a, b) = (m00, m01) on the bit-0 side and (m11, m10) on the bit-1 side
-template <int NV>
-__device__ __forceinline__ void lane_op(float2 (&R)[NV], float2 (&I)[NV], const QsvOp &op, const float *m0,
-                                        const float *m1, bool thread_ok, int lanebit, int lane) {
-    const int mine = (lane >> lanebit) & 1;
-    const int xm = 1 << lanebit;
-    const int cm_reg = op.cm_reg;
-    const bool uni = op.kind == QSV_K_UNI, ctrl = op.kind == QSV_K_CTRL, cc = op.cm_c;
-    const float a0r = mine ? m0[6] : m0[0], a0i = mine ? m0[7] : m0[1];
-    const float b0r = mine ? m0[4] : m0[2], b0i = mine ? m0[5] : m0[3];
-    const float a1r = mine ? m1[6] : m1[0], a1i = mine ? m1[7] : m1[1];
-    const float b1r = mine ? m1[4] : m1[2], b1i = mine ? m1[5] : m1[3];
-#pragma unroll
-    for (int r = 0; r < NV; r++) {
-        float2 oR, oI;
-        oR.x = __shfl_xor_sync(0xffffffffu, R[r].x, xm);
-        oR.y = __shfl_xor_sync(0xffffffffu, R[r].y, xm);
-        oI.x = __shfl_xor_sync(0xffffffffu, I[r].x, xm);
-        oI.y = __shfl_xor_sync(0xffffffffu, I[r].y, xm);
-        const bool sy = !uni && thread_ok && (r & cm_reg) == cm_reg, sx = sy && !cc;
-        // unselected pairs of a controlled op use M0 = identity: (a, b) = (1, 0) leaves the amplitude's
-        // value unchanged, so the arithmetic runs branch-free on every lane
-        const float u0r = ctrl ? 1.f : a0r, u0i = ctrl ? 0.f : a0i, v0r = ctrl ? 0.f : b0r, v0i = ctrl ? 0.f : b0i;
-        const float2 ar = make_float2(sx ? a1r : u0r, sy ? a1r : u0r);
-        const float2 ai = make_float2(sx ? a1i : u0i, sy ? a1i : u0i);
-        const float2 br = make_float2(sx ? b1r : v0r, sy ? b1r : v0r);
-        const float2 bi = make_float2(sx ? b1i : v0i, sy ? b1i : v0i);
-        float2 t = __fmul2_rn(make_float2(-bi.x, -bi.y), oI);
-        t = __ffma2_rn(br, oR, t);
-        t = __ffma2_rn(make_float2(-ai.x, -ai.y), I[r], t);
-        const float2 yr = __ffma2_rn(ar, R[r], t);
-        float2 u = __fmul2_rn(bi, oR);
-        u = __ffma2_rn(br, oI, u);
-        u = __ffma2_rn(ai, R[r], u);
-        const float2 yi = __ffma2_rn(ar, I[r], u);
-        R[r] = yr;
-        I[r] = yi;
-    }
-}
-
 // ---------------------------------------------------------------- shared building blocks
-// lane update y = a*own + b*oth on two packed pairs (the lane_op arithmetic with hoisted coefficients)
-__device__ __forceinline__ void lane_lin(float2 &R, float2 &I, const float2 oR, const float2 oI, const float2 ar,
-                                         const float2 ai, const float2 nai, const float2 br, const float2 bi,
-                                         const float2 nbi) {
-    float2 t = __fmul2_rn(nbi, oI);
-    t = __ffma2_rn(br, oR, t);
-    t = __ffma2_rn(nai, I, t);
-    const float2 yr = __ffma2_rn(ar, R, t);
-    float2 u = __fmul2_rn(bi, oR);
-    u = __ffma2_rn(br, oI, u);
-    u = __ffma2_rn(ai, R, u);
-    const float2 yi = __ffma2_rn(ar, I, u);
-    R = yr;
-    I = yi;
-}
-__device__ __forceinline__ void shfl4(const float2 &R, const float2 &I, float2 &oR, float2 &oI, int xm) {
-    oR.x = __shfl_xor_sync(0xffffffffu, R.x, xm);
-    oR.y = __shfl_xor_sync(0xffffffffu, R.y, xm);
-    oI.x = __shfl_xor_sync(0xffffffffu, I.x, xm);
-    oI.y = __shfl_xor_sync(0xffffffffu, I.y, xm);
-}
 // pair_apply with the matrix class fixed at compile time
 template <int CLS>
 __device__ __forceinline__ void pair_t(float &x0r, float &x0i, float &x1r, float &x1i, const float *m) {
@@ -312,7 +251,7 @@ __device__ __forceinline__ void pair_t(float &x0r, float &x0i, float &x1r, float
 
 // ---------------------------------------------------------------- one dispatch per op
 // The interpreter's fast paths: a uniform switch per op selects a tight loop (coefficients hoisted, no
-// per-pair selects). Same values as comp_op / lane_op (forms that skip work skip exact-zero terms or
+// per-pair selects). Same values as comp_op (forms that skip work skip exact-zero terms or
 // unselected pairs only).
 template <int NV, int CLS, bool CTRL>
 __device__ __forceinline__ void comp_loop(float2 (&R)[NV], float2 (&I)[NV], const float *m, int cm_reg, bool tok) {

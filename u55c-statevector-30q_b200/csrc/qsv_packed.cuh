@@ -18,7 +18,6 @@ __device__ __forceinline__ p2 pk(float lo, float hi) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }
-__device__ __forceinline__ p2 splat(float a) { return pk(a, a); }
 __device__ __forceinline__ void unpk(p2 a, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a)); }
 __device__ __forceinline__ p2 flip(p2 a) {       // exchange the halves
     float lo, hi;
