@@ -294,7 +294,9 @@ __device__ __forceinline__ void jit_comp(p2 (&R)[NV], p2 (&I)[NV], const p2 *C, 
     };
     float a[8], b[8];                                  // the selected slots' matrix, the others'
     constexpr int CA = UNI ? CLS0 : CLS1;
-    if constexpr (CA != QSV_M_XSWAP && CA != QSV_M_IDENT) mat(C, a);
+    // an exchange or the identity has code of its own and no coefficients, except as one of two matrices to choose
+    // between: both of those are applied as dense ones, whatever their class
+    if constexpr ((!UNI && !CTRL) || (CA != QSV_M_XSWAP && CA != QSV_M_IDENT)) mat(C, a);
     if constexpr (!UNI && !CTRL) mat(C + 12, b);
 #pragma unroll
     for (int r = 0; r < NV; r++) {
