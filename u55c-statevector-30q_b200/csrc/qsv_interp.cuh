@@ -132,6 +132,23 @@ __device__ __forceinline__ void phase_op(p2 (&R)[NV], p2 (&I)[NV], p2 ar, p2 ai,
     }
 }
 
+// The same on the high halves alone (a phase on tile bit 0, or under a control there). The low halves stay as they are:
+// a packed factor of (1, 0) for them would spread an infinity or a NaN from one part of an amplitude to the other. (That
+// form was 0.9 % faster on a 27-qubit random circuit and 1.9 % on a transform; straight-line code for each slot mask,
+// here or beside phase_op, was no faster than this.)
+template <int NV>
+__device__ __forceinline__ void phase_hi_op(p2 (&R)[NV], p2 (&I)[NV], const MatP &M, uint32_t sel) {
+    const float dr = hi_of(M.c[0]), di = hi_of(M.c[1]);
+#pragma unroll
+    for (int r = 0; r < NV; r++)
+        QSV_SEL {
+            const HalvesP x(R[r], I[r]);
+            float yr, yi;
+            diag_own(yr, yi, dr, di, x.rh, x.ih);
+            x.put(R[r], I[r], yr, yi);
+        }
+}
+
 // Tile-bit-0 target: the two halves of every slot are a pair; each half is own, the other half its partner.
 __device__ __forceinline__ OwnP first_own(const MatP &M) { return OwnP{M.c[0], M.c[1], M.c[2], M.c[3], M.c[4], M.c[5]}; }
 template <int NV>
@@ -220,6 +237,8 @@ __device__ __forceinline__ void apply_op_p(const HdrP &h, const QsvIOp *op, p2 (
     } else if (path >= QSV_P_LANE_DENSE) {
         if (path <= QSV_P_LANE_MUX) {
             lane_op_p<NV>(R, I, h, M, op, tok, lane);
+        } else if (path == QSV_P_PHASE_HI) {
+            if (tok) phase_hi_op<NV>(R, I, M, sel);
         } else if (path == QSV_P_COMP_DENSE) {
             comp_pass<NV>(R, I, first_own(M), 0xffffffffu);
         } else if (path == QSV_P_BASE_DIAG) {

@@ -24,7 +24,7 @@ typedef unsigned long long p2;      // two packed floats: low half = amplitude w
 //   own layout (tile-bit-0 target: low half, high half): a.re a.im -a.im b.re b.im -b.im with y = a own +
 //     b other, (a, b) = (m00, m01) on the low half and (m11, m10) on the high half
 //   phase layout: a.re a.im -a.im for the selected amplitudes (path BASE_DIAG: then the same for amplitudes
-//     with the target bit set)
+//     with the target bit set; path PHASE_HI: the high halves alone count)
 // A path is a group (path >> 2) and, for register-bit targets, the register bit (path & 3).
 enum : int {
     QSV_G_DENSE_R0 = 0,       // every pair; m00 real (its imaginary part an exact zero, as in every U3)
@@ -46,6 +46,7 @@ enum : int {
     QSV_P_COMP_MUX = 43,
     QSV_P_BASE_DIAG = 44,     // every slot, by a bit of the thread base
     QSV_P_SKIP = 45,
+    QSV_P_PHASE_HI = 46,      // high halves of the slots in sel, where tok: a phase under tile bit 0
 };
 struct alignas(16) QsvIOp {
     uint32_t cm_thr;          // thread-base bits that must be set (tok)
@@ -89,13 +90,14 @@ QSV_HD void iop_header(const Op &op, int slots, IOp &o) {
     const bool ctrl = op.kind == QSV_K_CTRL, mux = op.kind == QSV_K_MUX;
     const bool swap = v == QSV_V_UNI_SWAP || v == QSV_V_CTRL_SWAP || v == QSV_V_CTRL_SWAP_SEL;
     const bool half = v == QSV_V_MUX && ctrl;        // controlled, tile bit 0 among the controls
+    const bool high = iop_phase(op) && (comp || half);       // ... or the target: only the high halves are touched
     int path = QSV_P_SKIP, flag = 0;
     uint32_t thr = op.cm_thr, tmask = 0;
     int rm = op.cm_reg;
     if (v == QSV_V_SKIP) {
         path = QSV_P_SKIP;
     } else if (iop_phase(op) || (comp && op.cls == QSV_M_DIAG && !mux)) {
-        path = QSV_G_PHASE << 2;
+        path = high ? QSV_P_PHASE_HI : QSV_G_PHASE << 2;
         if (reg) rm |= 1 << rb;
         else if (!comp) thr |= 1u << op.tbit;
     } else if (v == QSV_V_UNI_DIAG) {
@@ -119,8 +121,9 @@ QSV_HD void iop_header(const Op &op, int slots, IOp &o) {
         path = (g << 2) + rb;
     }
     uint32_t sel = 0;
+    const int need = high ? rm : op.cm_reg;
     for (int r = 0; r < slots; r++)
-        if ((r & op.cm_reg) == op.cm_reg) sel |= 1u << r;
+        if ((r & need) == need) sel |= 1u << r;
     o.cm_thr = thr;
     o.path = (uint32_t)path;
     o.sel = sel;
@@ -140,7 +143,7 @@ QSV_HD p2 iop_coef(const QsvOp &op, int e) {
         const int i = (k % 3) == 0 ? 0 : 1;
         float lo, hi;
         if (comp) { lo = m[i]; hi = m[6 + i]; }
-        else { lo = hi = m[(one ? 6 : 0) + i]; if (op.kind == QSV_K_CTRL && op.cm_c) lo = i ? 0.f : 1.f; }
+        else lo = hi = m[(one ? 6 : 0) + i];
         return (k % 3) == 2 ? pack2(-lo, -hi) : pack2(lo, hi);
     }
     // the matrix of this half of the record: a = the one the op applies (M1 under controls), b = M0 (MUX)
