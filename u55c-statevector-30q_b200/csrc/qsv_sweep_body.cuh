@@ -276,6 +276,9 @@ __device__ __forceinline__ void sweep_pipeline(typename Body::Amp *__restrict__ 
         Body::template expand_phases<RB, WB>(sops, P, tid, NC);
         named_bar_sync(1, NC);
     }
+    // the limit of the waits below counts from the end of the work before this sweep: that work may be long (a kernel
+    // of the caller's that lets its dependents start early)
+    grid_wait();
     if constexpr (IL != 0) {
         static_assert(G == 1, "interleaved phases run one consumer group");
         // tiles j0 and j0 + 1 (slots u = 0, 1): phase p of both, then phase p + 1 of both. Every consumer
