@@ -19,6 +19,7 @@
 #include "qsv_interp.cuh"
 #include "qsv_ops.cuh"
 #include "qsv_planner.h"
+#include "qsv_side.h"
 
 namespace qsv {
 
@@ -136,37 +137,9 @@ struct Batch {
     int group_off[QSV_KW_MAX + 1] = {0}, group_cnt[QSV_KW_MAX + 1] = {0};
     size_t off_phases = 0, off_ops = 0, bytes = 0;
     bool finalized = false;
-    // Streams of their own for all but one of the qubit counts, and the events that tie them to the caller's
-    // stream (made with the upload, on its device).
-    static constexpr int kSide = QSV_KW_MAX - 10;
-    cudaStream_t side[kSide] = {};
-    cudaEvent_t fork = nullptr, joined[kSide] = {};
-    int side_dev = -1;
+    // streams of their own for all but one of the qubit counts (taken with the upload, on its device)
+    SideStreams *side = nullptr;
 };
-
-static void batch_drop_streams(Batch *b) {
-    for (int k = 0; k < Batch::kSide; k++) {
-        if (b->side[k]) cudaStreamDestroy(b->side[k]);
-        if (b->joined[k]) cudaEventDestroy(b->joined[k]);
-        b->side[k] = nullptr;
-        b->joined[k] = nullptr;
-    }
-    if (b->fork) cudaEventDestroy(b->fork);
-    b->fork = nullptr;
-    b->side_dev = -1;
-}
-
-static void batch_make_streams(Batch *b) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || b->side_dev == dev) return;
-    batch_drop_streams(b);
-    bool ok = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess;
-    for (int k = 0; ok && k < Batch::kSide; k++)
-        ok = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) == cudaSuccess &&
-             cudaEventCreateWithFlags(&b->joined[k], cudaEventDisableTiming) == cudaSuccess;
-    if (ok) b->side_dev = dev;
-    else batch_drop_streams(b);          // the launch runs the qubit counts one after the other
-}
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -232,7 +205,17 @@ cudaError_t batch_upload(Batch *b, void *ws, cudaStream_t stream) {
     batch_finalize(b);
     int groups = 0;
     for (int n = 10; n <= QSV_KW_MAX; n++) groups += b->group_cnt[n] > 0;
-    if (groups > 1) batch_make_streams(b);
+    if (groups > 1) {
+        static_assert(SideStreams::kMax >= QSV_KW_MAX - 10, "a side stream for all but one of the qubit counts");
+        int dev = 0;
+        const cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        if (b->side && b->side->dev != dev) {
+            side_give(b->side);
+            b->side = nullptr;
+        }
+        if (!b->side) b->side = side_take();     // none: the launch runs the qubit counts one after the other
+    }
     char *base = static_cast<char *>(ws);
     cudaError_t e = cudaSuccess;
     if (!b->items.empty())
@@ -264,17 +247,17 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
     e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     for (int n = 10; n <= QSV_KW_MAX; n++) groups += b->group_cnt[n] > 0;
-    const bool beside = groups > 1 && b->side_dev == dev;
-    if (beside && (e = cudaEventRecord(b->fork, stream)) != cudaSuccess) return e;
+    const SideStreams *side = groups > 1 && b->side && b->side->dev == dev ? b->side : nullptr;
+    if (side && (e = cudaEventRecord(side->fork, stream)) != cudaSuccess) return e;
     cudaError_t bad = cudaSuccess;
     for (int n = QSV_KW_MAX; n >= 10 && bad == cudaSuccess; n--) {
         const int cnt = b->group_cnt[n];
         if (!cnt) continue;
         const BatchItem *it = items + b->group_off[n];
         cudaStream_t st = stream;
-        if (beside && *launches > 0) {
-            st = b->side[k];
-            bad = cudaStreamWaitEvent(st, b->fork, 0);
+        if (side && *launches > 0) {
+            st = side->stream[k];
+            bad = cudaStreamWaitEvent(st, side->fork, 0);
             if (bad != cudaSuccess) break;
         }
         switch (n) {
@@ -284,8 +267,8 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
             default: bad = dev::launch_batch_t<10, 2, 2, 3>(it, cnt, phases, ops, status, nsm, st); break;
         }
         if (st != stream) {              // the caller's stream goes on after the side stream, also on an error
-            cudaError_t j = cudaEventRecord(b->joined[k], st);
-            if (j == cudaSuccess) j = cudaStreamWaitEvent(stream, b->joined[k], 0);
+            cudaError_t j = cudaEventRecord(side->joined[k], st);
+            if (j == cudaSuccess) j = cudaStreamWaitEvent(stream, side->joined[k], 0);
             if (bad == cudaSuccess) bad = j;
             k++;
         }
@@ -296,7 +279,7 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
 
 Batch *batch_new() { return new Batch(); }
 void batch_free(Batch *b) {
-    batch_drop_streams(b);
+    side_give(b->side);
     delete b;
 }
 int batch_size(const Batch *b) { return (int)b->circs.size(); }
