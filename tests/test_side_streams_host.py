@@ -1,4 +1,5 @@
-"""Side streams (csrc/qsv_side.cpp) over a fake CUDA runtime, on the host: what a failed call leaves behind."""
+"""Side streams (csrc/qsv_side.cpp) over a fake CUDA runtime, on the host: what a failed call leaves behind, and which
+streams they can be tied to while something is being captured."""
 import ctypes
 import os
 import subprocess
@@ -11,9 +12,11 @@ from qsv_b200 import build
 FAKE = r"""
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <map>
 #include "qsv_side.h"
 static int live_streams = 0, live_events = 0, made = 0, fail_at = -1, device = 0;
 static cudaError_t last = cudaSuccess;
+static std::map<cudaStream_t, int> captures;     // graph each captured stream belongs to (-1: cannot be asked)
 static cudaError_t step() {
     if (made++ == fail_at) return last = cudaErrorMemoryAllocation;
     return cudaSuccess;
@@ -33,6 +36,17 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t *v, unsigned) {
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { live_streams--; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { live_events--; return cudaSuccess; }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus *st, unsigned long long *id, cudaGraph_t *,
+                                     const cudaGraphNode_t **, size_t *) {
+    const auto c = captures.find(s);
+    if (c != captures.end() && c->second < 0) return last = cudaErrorStreamCaptureImplicit;
+    *st = c == captures.end() ? cudaStreamCaptureStatusNone : cudaStreamCaptureStatusActive;
+    *id = c == captures.end() ? 0 : c->second;
+    return cudaSuccess;
+}
+void fake_capture(void *s, int graph) { if (graph) captures[(cudaStream_t)s] = graph; else captures.erase((cudaStream_t)s); }
+void *side_stream(void *s, int k) { return ((qsv::SideStreams *)s)->stream[k]; }
+int joins(void *s, int count, void *stream) { return qsv::side_joins((qsv::SideStreams *)s, count, (cudaStream_t)stream); }
 void fake_reset(int fail, int dev) { made = 0; fail_at = fail; device = dev; last = cudaSuccess; }
 int fake_made() { return made; }
 int fake_live() { return live_streams + live_events; }
@@ -54,6 +68,10 @@ def side(tmp_path_factory):
     lib = ctypes.CDLL(str(so))
     lib.take.restype = ctypes.c_void_p
     lib.give.argtypes = [ctypes.c_void_p]
+    lib.side_stream.restype = ctypes.c_void_p
+    lib.side_stream.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    lib.fake_capture.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    lib.joins.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
     return lib
 
 
@@ -69,3 +87,23 @@ def test_a_failed_call_leaves_no_error_and_no_streams(side):
         assert side.take() is None
         assert side.fake_last() == 0, f"call {k} left its error for the next launch to report"
         assert side.fake_live() == before
+
+
+def test_streams_in_another_capture_are_not_joined(side):
+    side.fake_reset(-1, 0)
+    s = side.take()
+    caller, last = 0x77, side.side_stream(s, 2)
+    assert side.joins(s, 3, caller)
+    side.fake_capture(caller, 5)
+    assert side.joins(s, 3, caller)              # free side streams join the caller's capture
+    side.fake_capture(last, 5)
+    assert side.joins(s, 3, caller)              # and are in it at its next launch
+    side.fake_capture(caller, 0)
+    assert not side.joins(s, 3, caller) and side.joins(s, 2, caller)
+    side.fake_capture(caller, 6)
+    assert not side.joins(s, 3, caller)
+    side.fake_capture(last, 0)
+    side.fake_capture(caller, -1)
+    assert not side.joins(s, 1, caller) and side.fake_last() == 0
+    side.fake_capture(caller, 0)
+    side.give(s)

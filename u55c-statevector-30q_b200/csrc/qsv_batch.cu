@@ -248,6 +248,7 @@ cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *
     if (e != cudaSuccess) return e;
     for (int n = 10; n <= QSV_KW_MAX; n++) groups += b->group_cnt[n] > 0;
     const SideStreams *side = groups > 1 && b->side && b->side->dev == dev ? b->side : nullptr;
+    if (side && !side_joins(side, groups - 1, stream)) side = nullptr;
     if (side && (e = cudaEventRecord(side->fork, stream)) != cudaSuccess) return e;
     cudaError_t bad = cudaSuccess;
     for (int n = QSV_KW_MAX; n >= 10 && bad == cudaSuccess; n--) {

@@ -37,4 +37,20 @@ void side_give(SideStreams *s) {
     if (s) destroy(s);
 }
 
+static bool capture_of(cudaStream_t stream, cudaStreamCaptureStatus *status, unsigned long long *id) {
+    *id = 0;
+    return cudaStreamGetCaptureInfo(stream, status, id) == cudaSuccess;
+}
+
+bool side_joins(const SideStreams *s, int count, cudaStream_t stream) {
+    cudaStreamCaptureStatus own, st;
+    unsigned long long own_id, id;
+    bool ok = capture_of(stream, &own, &own_id) && own != cudaStreamCaptureStatusInvalidated;
+    for (int k = 0; ok && k < count; k++)
+        ok = capture_of(s->stream[k], &st, &id) &&
+             (st == cudaStreamCaptureStatusNone || (st == own && id == own_id));
+    if (!ok) cudaGetLastError();     // (the legacy stream cannot be asked during a capture elsewhere)
+    return ok;
+}
+
 }  // namespace qsv

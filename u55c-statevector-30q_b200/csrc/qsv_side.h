@@ -15,5 +15,9 @@ struct SideStreams {
 // no error is left behind for its next launch to report.
 SideStreams *side_take();
 void side_give(SideStreams *s);
+// Whether work on the first `count` streams of s can be tied to the caller's stream: they are captured into the same
+// graph as it is, or neither it nor they are captured. (A side stream that a launch has brought into a capture stays in
+// it until the capture ends; work of other streams must not meet it there.)
+bool side_joins(const SideStreams *s, int count, cudaStream_t stream);
 
 }  // namespace qsv
