@@ -1,5 +1,5 @@
-"""Side streams (csrc/qsv_side.cpp) over a fake CUDA runtime, on the host: what a failed call leaves behind, and which
-streams they can be tied to while something is being captured."""
+"""Side streams (csrc/qsv_side.cpp) over a fake CUDA runtime, on the host: what a failed call leaves behind, which
+streams they can be tied to while something is being captured, and that sets are made once, kept and bounded."""
 import ctypes
 import os
 import subprocess
@@ -44,6 +44,10 @@ cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus *st
     *id = c == captures.end() ? 0 : c->second;
     return cudaSuccess;
 }
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus *st) {
+    *st = captures.count(s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
 void fake_capture(void *s, int graph) { if (graph) captures[(cudaStream_t)s] = graph; else captures.erase((cudaStream_t)s); }
 void *side_stream(void *s, int k) { return ((qsv::SideStreams *)s)->stream[k]; }
 int joins(void *s, int count, void *stream) { return qsv::side_joins((qsv::SideStreams *)s, count, (cudaStream_t)stream); }
@@ -51,6 +55,7 @@ void fake_reset(int fail, int dev) { made = 0; fail_at = fail; device = dev; las
 int fake_made() { return made; }
 int fake_live() { return live_streams + live_events; }
 int fake_last() { return (int)last; }
+int kept() { return qsv::kSideKept; }
 void *take() { return qsv::side_take(); }
 void give(void *s) { qsv::side_give((qsv::SideStreams *)s); }
 }
@@ -68,6 +73,7 @@ def side(tmp_path_factory):
     lib = ctypes.CDLL(str(so))
     lib.take.restype = ctypes.c_void_p
     lib.give.argtypes = [ctypes.c_void_p]
+    lib.kept.restype = ctypes.c_int
     lib.side_stream.restype = ctypes.c_void_p
     lib.side_stream.argtypes = [ctypes.c_void_p, ctypes.c_int]
     lib.fake_capture.argtypes = [ctypes.c_void_p, ctypes.c_int]
@@ -107,3 +113,47 @@ def test_streams_in_another_capture_are_not_joined(side):
     assert not side.joins(s, 1, caller) and side.fake_last() == 0
     side.fake_capture(caller, 0)
     side.give(s)
+
+
+def test_sets_are_handed_out_again_and_bounded(side):
+    side.fake_reset(-1, 20)                      # a device of its own
+    start = side.fake_live()
+    s = side.take()
+    one = side.fake_live() - start
+    side.give(s)
+    side.fake_reset(-1, 20)
+    for _ in range(50):
+        s = side.take()
+        side.give(s)
+    assert side.fake_made() == 0 and side.fake_live() - start == one
+    # never the same set twice at a time; not another device's
+    some = [side.take() for _ in range(2 * side.kept())]
+    assert len(set(some)) == len(some)
+    for s in some:
+        side.give(s)
+    assert side.fake_live() - start == side.kept() * one
+    side.fake_reset(-1, 21)
+    other = side.take()
+    assert other not in some and side.fake_made() > 0
+    side.give(other)
+
+
+def test_captured_sets_stay_until_their_capture_ends(side):
+    side.fake_reset(-1, 22)
+    start = side.fake_live()
+    held = side.take()
+    one = side.fake_live() - start
+    side.fake_capture(side.side_stream(held, 1), 9)
+    side.give(held)
+    s = side.take()
+    assert s != held
+    some = [s] + [side.take() for _ in range(side.kept())]
+    assert held not in some
+    for s in some:
+        side.give(s)
+    assert side.fake_live() - start == side.kept() * one
+    side.fake_capture(side.side_stream(held, 1), 0)
+    got = [side.take() for _ in range(side.kept())]
+    assert held in got and side.fake_live() - start == side.kept() * one
+    for s in got:
+        side.give(s)
