@@ -126,10 +126,14 @@ QSV_API size_t qsv_batch_workspace_bytes(qsv_batch *batch);
 QSV_API int qsv_batch_upload(qsv_batch *batch, void *workspace, size_t bytes, void *stream);
 QSV_API int qsv_batch_launch(qsv_batch *batch, void *workspace, size_t bytes, void *stream);
 
-/* Host-side decode of a segment into the sweep plan the engine launches, for inspection and tests.
- * Writes at most `cap` int32 words to `out` (layout in csrc/qsv_plan.h, qsv_plan_serialize) and returns
- * the number of words of the full plan, or a negative error code. Pure host code, no device work. */
+/* Host-side decode of a segment into the sweeps the engine launches, as its specialised kernels run them, for
+ * inspection and tests. Writes at most `cap` int32 words to `out` (layout in csrc/qsv_planner.h, serialize) and
+ * returns the number of words of the full plan, or a negative error code. Pure host code, no device work. */
 QSV_API int qsv_plan_segment(const int32_t *seg, size_t nwords, int n, int32_t *out, size_t cap);
+
+/* The same sweeps as the phase interpreter runs them (every sweep without a specialised kernel): fewer register
+ * bits, so other phases, slots, control splits and layouts. Words as qsv_plan_segment's. */
+QSV_API int qsv_plan_interp(const int32_t *seg, size_t nwords, int n, int32_t *out, size_t cap);
 
 /* The streaming form of the same sweeps (no reference counterpart): how the streaming interpreter and the
  * group-type library run them. Writes at most `cap` int32 words: the sweep count, then per sweep kw,

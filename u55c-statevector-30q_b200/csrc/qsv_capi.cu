@@ -128,7 +128,7 @@ int qsv_inject_skip_load(int count) {
     return QSV_OK;
 }
 
-int qsv_plan_segment(const int32_t *seg, size_t nwords, int n, int32_t *out, size_t cap) {
+static int plan_words(const int32_t *seg, size_t nwords, int n, int32_t *out, size_t cap, bool interp) {
     if (n < QSV_N_MIN || n > QSV_N_MAX) return fail(QSV_ERR_INVALID_ARG, "n out of [10, 34]");
     std::vector<qsv::PhysPass> passes;
     std::string err;
@@ -136,9 +136,17 @@ int qsv_plan_segment(const int32_t *seg, size_t nwords, int n, int32_t *out, siz
     if (rc) return fail(rc, err);
     std::vector<QsvSweep> sweeps;
     const int kw = n < QSV_KW_MAX ? n : QSV_KW_MAX;
-    rc = qsv::build_sweeps<QsvOp>(passes, n, kw, g_lo_merge, sweeps, err);
+    rc = qsv::build_sweeps<QsvOp>(passes, n, kw, g_lo_merge, sweeps, err, interp);
     if (rc) return fail(rc, err);
-    return qsv::serialize(sweeps, out, cap);
+    return qsv::serialize(sweeps, out, cap, interp);
+}
+
+int qsv_plan_segment(const int32_t *seg, size_t nwords, int n, int32_t *out, size_t cap) {
+    return plan_words(seg, nwords, n, out, cap, false);
+}
+
+int qsv_plan_interp(const int32_t *seg, size_t nwords, int n, int32_t *out, size_t cap) {
+    return plan_words(seg, nwords, n, out, cap, true);
 }
 
 int qsv_plan_stream(const int32_t *seg, size_t nwords, int n, int32_t *out, size_t cap) {

@@ -698,12 +698,13 @@ int serialize_stream(const std::vector<QsvSweep> &sw, int32_t *out, size_t cap) 
     return (int)w.size();
 }
 
-int serialize(const std::vector<QsvSweep> &sw, int32_t *out, size_t cap) {
+int serialize(const std::vector<QsvSweep> &sw, int32_t *out, size_t cap, bool interp) {
     std::vector<int32_t> w;
     w.push_back((int32_t)sw.size());
     for (const QsvSweep &s : sw) {
         int rb = 0, wb = 0;
-        layout_for_kw(s.kw, &rb, &wb);
+        if (interp) layout_interp(s.kw, &rb, &wb);
+        else layout_for_kw(s.kw, &rb, &wb);
         w.push_back(s.kw); w.push_back(s.lo); w.push_back(s.nh);
         for (int i = 0; i < QSV_KW_MAX; i++) w.push_back(i < s.nh ? s.H[i] : -1);
         w.push_back(s.tma_rank);
@@ -732,6 +733,7 @@ int serialize(const std::vector<QsvSweep> &sw, int32_t *out, size_t cap) {
             for (int e = 0; e < 8; e++) w.push_back(b[e]);
         }
     }
+    for (const QsvSweep &s : sw) w.push_back(s.tma_xbits);
     if (out) std::memcpy(out, w.data(), sizeof(int32_t) * std::min(cap, w.size()));
     return (int)w.size();
 }

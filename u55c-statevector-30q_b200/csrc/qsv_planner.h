@@ -67,7 +67,11 @@ int plan_stream(QsvSweep &sw, std::string &err);
 // Flatten streaming plans (plan_stream) into int32 words: sweeps; per sweep kw, ngroups, nops, then per group
 // q0 q1 q2 op_begin op_end, then per op tbit slot variant cmask cm_reg cm_thr kind.
 int serialize_stream(const std::vector<QsvSweep> &sw, int32_t *out, size_t cap);
-// Flatten a plan into int32 words (layout documented in qsv_b200.h / the planner tests).
-int serialize(const std::vector<QsvSweep> &sw, int32_t *out, size_t cap);
+// Flatten a plan into int32 words; interp: sweeps planned for the phase interpreter. Words: sweeps; per sweep kw, lo,
+// nh, H (QSV_KW_MAX, then -1), tma_rank, tdim_free and tdim_box (QSV_TMA_MAX_RANK each, then -1), swz, nphases, nops, per
+// phase reg_bits (QSV_RB_MAX, then -1), lane_bits[2], warp_bits (QSV_WB_MAX, then -1), op_begin, op_end, lane_lo[3], per
+// op tbit, slot, cmask, cls0, cls1, kind, cls, cm_reg, cm_c, cm_thr, variant, m0, m1 (8 floats each); after all sweeps
+// tma_xbits of each.
+int serialize(const std::vector<QsvSweep> &sw, int32_t *out, size_t cap, bool interp = false);
 
 }  // namespace qsv

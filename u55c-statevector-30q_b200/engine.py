@@ -73,6 +73,7 @@ def load(path=LIB_PATH):
         "qsv_inject_skip_load": ([ctypes.c_int], I32),
         "qsv_jit_prepare": ([P, SZ, ctypes.c_int], I32),
         "qsv_jit_wait": ([], I32),
+        "qsv_plan_interp": ([P, SZ, ctypes.c_int, P, SZ], I32),
         "qsv_plan_stream": ([P, SZ, ctypes.c_int, P, SZ], I32),
         "qsv_jit_prepare_library": ([P, P, P, ctypes.c_int], I32),
         "qsv_jit_info": ([P, ctypes.c_int], I32),
@@ -95,8 +96,8 @@ def exported_symbols():
     return ["qsv_version", "qsv_last_error", "qsv_run_segment", "qsv_remap", "qsv_zero_state",
             "qsv_reduce_scratch_bytes", "qsv_reduce_f64", "qsv_reduce_f64_noalloc", "qsv_chunk_probs_f64",
             "qsv_sample_f64",
-            "qsv_plan_segment", "qsv_plan_stream", "qsv_device_status", "qsv_take_launch_count", "qsv_set_lo_merge",
-            "qsv_set_layout13", "qsv_set_phase_lanes", "qsv_set_interp", "qsv_set_wait_limit_us",
+            "qsv_plan_segment", "qsv_plan_interp", "qsv_plan_stream", "qsv_device_status", "qsv_take_launch_count",
+            "qsv_set_lo_merge", "qsv_set_layout13", "qsv_set_phase_lanes", "qsv_set_interp", "qsv_set_wait_limit_us",
             "qsv_inject_skip_load", "qsv_batch_new", "qsv_batch_free", "qsv_batch_add",
             "qsv_batch_workspace_bytes", "qsv_batch_upload", "qsv_batch_launch", "qsv_set_jit", "qsv_jit_prepare",
             "qsv_jit_wait", "qsv_jit_prepare_library", "qsv_jit_info", "qsv_hbm_copy"]
@@ -223,16 +224,25 @@ def sample_f64(state, uniforms, scratch=None, stream=None):
     return out
 
 
-def plan_segment(seg, n):
-    """Decode a segment into the engine's sweep plan (host only): list of dicts."""
-    L = load()
+def _plan(fn, seg, n):
     w = np.ascontiguousarray(seg, dtype=np.int32)
-    need = L.qsv_plan_segment(w.ctypes.data_as(ctypes.c_void_p), w.size, n, None, 0)
+    need = fn(w.ctypes.data_as(ctypes.c_void_p), w.size, n, None, 0)
     if need < 0:
         _check(need)
     buf = np.zeros(need, dtype=np.int32)
-    L.qsv_plan_segment(w.ctypes.data_as(ctypes.c_void_p), w.size, n, buf.ctypes.data_as(ctypes.c_void_p), need)
+    fn(w.ctypes.data_as(ctypes.c_void_p), w.size, n, buf.ctypes.data_as(ctypes.c_void_p), need)
     return _parse_plan(buf, n)
+
+
+def plan_segment(seg, n):
+    """Decode a segment into the engine's sweeps as its specialised kernels run them (host only): list of dicts.
+    A tile is staged with ``1 << tma_xbits`` tensor-map boxes (``tma_rank`` 0: bulk copies)."""
+    return _plan(load().qsv_plan_segment, seg, n)
+
+
+def plan_interp(seg, n):
+    """The same sweeps as the phase interpreter runs them (host only): list of dicts."""
+    return _plan(load().qsv_plan_interp, seg, n)
 
 
 def plan_stream(seg, n):
@@ -295,6 +305,8 @@ def _parse_plan(w, n):
                             cm_reg=cm_reg, cm_c=cm_c, cm_thr=cm_thr & 0xFFFFFFFF, variant=variant, m0=m[:8], m1=m[8:]))
         sweeps.append(dict(kw=kw, lo=lo, H=H, window=list(range(lo)) + H, phases=phases, ops=ops,
                            tma_rank=rank, tdim_free=tfree, tdim_box=tbox, swizzled=bool(swz)))
+    for sw, x in zip(sweeps, w[pos:pos + len(sweeps)]):
+        sw["tma_xbits"] = int(x)
     return sweeps
 
 
