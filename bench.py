@@ -214,6 +214,18 @@ def precision_main(a):
 
 
 # ------------------------------------------------------------------ batched and served workloads
+def _build_library(mode, programs):
+    """The group-type library for the sweeps of the (segment, qubits) pairs that programs() lists, built before the
+    timed work, where the mode runs on it; its size and build time, or None."""
+    if mode != "library":
+        return None
+    from importlib import import_module
+    engine = import_module("qsv_b200.engine")
+    t0 = time.perf_counter()
+    big = programs()
+    return {"types": engine.jit_prepare_library(big) if big else 0, "build_s": round(time.perf_counter() - t0, 2)}
+
+
 def batched_main(a):
     """Batched: `count` circuits (qubits uniform in [10, 24], depths in [5, 40], U3 / CZ / Toffoli layers,
     circuit i seeded 3 + i) per replay of one captured CUDA graph, against the plain one-circuit-at-a-time
@@ -244,15 +256,8 @@ def batched_main(a):
             work_bytes += 16 << n
         else:
             work_bytes += sum(len(engine.plan_segment(seg, n)) for kind, seg in prog if kind == "segment") * (16 << n)
-    # the group-type library for the 13-qubit sweeps of the batch's larger circuits (one build before the
-    # timed work; the plain path below uses it too)
-    lib_info = None
-    if a.jit in ("auto", "library"):
-        t0 = time.perf_counter()
-        big = [(seg, n) for qc, (prog, fmap, n, npass) in zip(circs, progs) if n > batch.SMALL_MAX
-               for kind, seg in prog if kind == "segment"]
-        lib_info = {"types": engine.jit_prepare_library(big) if big else 0,
-                    "build_s": round(time.perf_counter() - t0, 2)}
+    lib_info = _build_library(a.jit, lambda: [(seg, n) for qc, (prog, fmap, n, npass) in zip(circs, progs)
+                                              if n > batch.SMALL_MAX for kind, seg in prog if kind == "segment"])
     br = batch.BatchRunner(streams=8, autotune=True)
     plan = br.prepare(circs, programs=progs)
     br.capture(plan)
@@ -356,16 +361,12 @@ def served_main(a):
             out.append(x)
         return out
 
-    # group-type libraries for the 13-qubit sweeps, from up to 400 sampled requests (a service builds them at
-    # start-up from its recent requests; both sides use them)
-    lib_info = None
-    if a.jit in ("auto", "library") and not a.compile_on_arrival:
-        t0 = time.perf_counter()
+    # the library of a service is built at start-up from up to 400 of its recent requests; both sides use it
+    def sampled():
         pick = base if len(base) <= 400 else [base[i] for i in np.random.default_rng(1).choice(len(base), 400,
                                                                                               replace=False)]
-        big = [(seg, r.n) for r in pick if r.n > 13 for seg in r.program]
-        lib_info = {"types": engine.jit_prepare_library(big) if big else 0,
-                    "build_s": round(time.perf_counter() - t0, 2)}
+        return [(seg, r.n) for r in pick if r.n > 13 for seg in r.program]
+    lib_info = None if a.compile_on_arrival else _build_library(a.jit, sampled)
     srv = serve.Server(budget_bytes=160e9, max_inflight=16, policy=a.policy,
                        compile_workers=workers if a.compile_on_arrival else 0)
     srv.warm()                      # compile workers started before the arrivals (service start-up)
