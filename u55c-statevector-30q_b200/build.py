@@ -17,7 +17,7 @@ SOURCES = ["qsv_capi.cu", "qsv_sweep.cu", "qsv_sweep_d.cu", "qsv_aux.cu", "qsv_b
 # device headers compiled into the library AND embedded in it for run-time (NVRTC) specialised kernels
 JIT_HEADERS = ["qsv_plan.h", "qsv_device.cuh", "qsv_ops.cuh", "qsv_packed.cuh", "qsv_sweep_body.cuh", "qsv_jit_ops.cuh",
                "qsv_stream.cuh"]
-HEADERS = JIT_HEADERS + ["qsv_planner.h", "qsv_interp.cuh", "qsv_iop.h", "qsv_launch.h", "qsv_side.h"]
+HEADERS = JIT_HEADERS + ["qsv_planner.h", "qsv_interp.cuh", "qsv_iop.h", "qsv_launch.h", "qsv_reduce.h", "qsv_side.h"]
 GEN = os.path.join(CSRC, "_gen", "qsv_jit_headers.inc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

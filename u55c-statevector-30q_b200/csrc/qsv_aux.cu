@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "qsv_device.cuh"
+#include "qsv_reduce.h"
 
 namespace qsv {
 namespace dev {
@@ -149,12 +150,13 @@ __global__ void set_amp0_kernel_d(double2 *state) { state[0] = make_double2(1.0,
 // amplitudes (256 threads, 16-byte loads, 16 in flight per thread: 16 float4 of two complex64 amplitudes each,
 // or 2 x 16 double2). A chunk's index bits are: bits in the 16-byte vector (complex64), 8 thread bits, 4 (5)
 // load bits, and the chunk number above. Per-bit sums of the load bits share one addition tree; a bit of the
-// thread or the chunk number selects whole-thread sums. Fixed summation order (deterministic).
+// thread or the chunk number selects whole-thread sums. The order of the sums depends on the qubit count and the
+// element type alone (reduce_grid), so results are equal bit for bit from run to run and on any number of SMs.
 // What bounds it: HBM. One read of the state, about 4 FP64 operations and 2 conversions per amplitude. With
 // the per-bit sums in a run-time-indexed array (local memory) a 30-qubit complex64 reduction took 2.61 ms,
 // half the HBM rate; now 1.23 ms (7.0 TB/s, reads only).
 #define RED_THREADS 256
-#define RED_CHUNK_BITS 13
+#define RED_CHUNK_BITS kRedChunkBits
 #define RED_HI 21                  // bits above a chunk: n <= 34
 
 // sums of |a|^2 over 16 loads: total, and the four load bits' sums (added to acc)
@@ -603,13 +605,6 @@ cudaError_t launch_set_amp0(void *state, int dtype, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-constexpr int reduce_bits_of(int n) {
-    int B = n - 10;
-    if (B < 13) B = 13;
-    if (B > n) B = n;
-    if (B > 25) B = 25;
-    return B;
-}
 int reduce_bits(int n) { return reduce_bits_of(n); }
 
 size_t reduce_scratch_bytes(int n, int chunk_bits) {
@@ -619,28 +614,11 @@ size_t reduce_scratch_bytes(int n, int chunk_bits) {
     return red > smp ? red : smp;
 }
 
-// The block partials of a reduction: `blocks` blocks of nout doubles. Up to 2^9 chunks (n = 22) every chunk is a
-// block of its own with the sums of its 13 bits; above, a grid of four blocks per SM takes chunks in turn and
-// keeps the sums of all n bits, as many blocks as fit the scratch that reduce_scratch_bytes declares.
-static void reduce_grid(int n, int nsm, int64_t *blocks, int *nout) {
-    const int B = reduce_bits(n);
-    const int64_t room = (1ll << (n - B)) * (B + 1);
-    if (n <= RED_CHUNK_BITS) { *blocks = 1; *nout = n + 1; return; }
-    if (n <= 22) { *blocks = 1ll << (n - RED_CHUNK_BITS); *nout = RED_CHUNK_BITS + 1; return; }
-    int64_t g = (int64_t)nsm * 4;
-    if (g > room / (n + 1)) g = room / (n + 1);
-    if (g > 1ll << (n - RED_CHUNK_BITS)) g = 1ll << (n - RED_CHUNK_BITS);
-    *blocks = g;
-    *nout = n + 1;
-}
-
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 template <class A>
-static cudaError_t launch_reduce_t(const A *state, int n, int nsm, double *out, double *partials, cudaStream_t stream) {
-    int64_t blocks;
-    int nout;
-    reduce_grid(n, nsm, &blocks, &nout);
+static cudaError_t launch_reduce_t(const A *state, int n, double *out, double *partials, cudaStream_t stream) {
+    const auto [blocks, nout] = reduce_grid(n);
     if (n < RED_CHUNK_BITS) dev::reduce_small_kernel<A><<<1, RED_THREADS, 0, stream>>>(state, n, partials);
     else if (aligned16(state))
         dev::reduce_chunks_kernel<A, true><<<(unsigned)blocks, RED_THREADS, 0, stream>>>(
@@ -654,9 +632,9 @@ static cudaError_t launch_reduce_t(const A *state, int n, int nsm, double *out, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_reduce(const void *state, int n, int dtype, double *out, void *scratch, int nsm, cudaStream_t stream) {
-    if (dtype) return launch_reduce_t((const double2 *)state, n, nsm, out, (double *)scratch, stream);
-    return launch_reduce_t((const float2 *)state, n, nsm, out, (double *)scratch, stream);
+cudaError_t launch_reduce(const void *state, int n, int dtype, double *out, void *scratch, cudaStream_t stream) {
+    if (dtype) return launch_reduce_t((const double2 *)state, n, out, (double *)scratch, stream);
+    return launch_reduce_t((const float2 *)state, n, out, (double *)scratch, stream);
 }
 
 // ---------------------------------------------------------------- reduction without caller scratch
@@ -669,10 +647,9 @@ cudaError_t launch_reduce(const void *state, int n, int dtype, double *out, void
 #define QSV_NOALLOC_N_MAX 34
 static __device__ __align__(256) double g_noalloc_reduce_scratch[QSV_NOALLOC_REDUCE_DOUBLES];
 
-constexpr long long noalloc_partials(int n) { return (1ll << (n - reduce_bits_of(n))) * (reduce_bits_of(n) + 1); }
 constexpr bool noalloc_fits_every_n() {
     for (int n = QSV_NOALLOC_N_MIN; n <= QSV_NOALLOC_N_MAX; n++)
-        if (noalloc_partials(n) > QSV_NOALLOC_REDUCE_DOUBLES) return false;
+        if (reduce_room(n) > QSV_NOALLOC_REDUCE_DOUBLES) return false;
     return true;
 }
 static_assert(noalloc_fits_every_n(), "the fixed reduction scratch must hold the partials of every supported n");
@@ -701,15 +678,14 @@ static cudaError_t noalloc_scratch_ptr(double **out) {
     return cudaSuccess;
 }
 
-cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *out, int nsm, cudaStream_t stream,
-                                  size_t *need) {
-    const size_t doubles = (size_t)noalloc_partials(n);
+cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *out, cudaStream_t stream, size_t *need) {
+    const size_t doubles = (size_t)reduce_room(n);
     *need = doubles * sizeof(double);
     if (doubles > QSV_NOALLOC_REDUCE_DOUBLES) return cudaErrorInvalidValue;
     double *scratch = nullptr;
     cudaError_t e = noalloc_scratch_ptr(&scratch);
     if (e != cudaSuccess) return e;
-    return launch_reduce(state, n, dtype, out, scratch, nsm, stream);
+    return launch_reduce(state, n, dtype, out, scratch, stream);
 }
 
 template <class A>

@@ -20,7 +20,7 @@ cudaError_t launch_remap(const void *src, void *dst, int n, const int32_t *perm,
                          cudaStream_t stream);
 cudaError_t launch_set_amp0(void *state, int dtype, cudaStream_t stream);
 cudaError_t launch_copy_probe(void *dst, const void *src, size_t bytes, int nsm, cudaStream_t stream);
-cudaError_t launch_reduce(const void *state, int n, int dtype, double *out, void *scratch, int nsm, cudaStream_t stream);
+cudaError_t launch_reduce(const void *state, int n, int dtype, double *out, void *scratch, cudaStream_t stream);
 cudaError_t launch_chunk_probs(const void *state, int n, int dtype, int cb, double *out, int nsm, cudaStream_t stream);
 cudaError_t launch_sample(const void *state, int n, int dtype, int cb, const double *uni, int shots, int64_t *out,
                           void *scratch, int nsm, cudaStream_t stream);
@@ -33,8 +33,7 @@ int batch_add(Batch *b, void *state, int n, int nseg, const int32_t *const *segs
 size_t batch_workspace_bytes(Batch *b);
 cudaError_t batch_upload(Batch *b, void *ws, cudaStream_t stream);
 cudaError_t batch_launch(Batch *b, void *ws, int nsm, cudaStream_t stream, int *launches);
-cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *out, int nsm, cudaStream_t stream,
-                                  size_t *need);
+cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *out, cudaStream_t stream, size_t *need);
 size_t noalloc_reduce_capacity();
 int jit_set_mode(int mode);
 int jit_mode();
@@ -305,7 +304,7 @@ int qsv_reduce_f64(const void *state, int n, int dtype, double *out_dev, void *s
     if (!dtype_ok(dtype)) return fail(QSV_ERR_UNSUPPORTED, "dtype must be QSV_C64 or QSV_C128");
     if (n < QSV_N_MIN || n > QSV_N_MAX) return fail(QSV_ERR_INVALID_ARG, "n out of [10, 34]");
     if (scratch_bytes < qsv_reduce_scratch_bytes(n)) return fail(QSV_ERR_SCRATCH, "scratch too small");
-    cudaError_t e = qsv::launch_reduce(state, n, dtype, out_dev, scratch, sm_count(), (cudaStream_t)stream);
+    cudaError_t e = qsv::launch_reduce(state, n, dtype, out_dev, scratch, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "reduce launch");
     t_launches += 2;
     return QSV_OK;
@@ -317,7 +316,7 @@ int qsv_reduce_f64_noalloc(const void *state, int n, int dtype, double *out_dev,
     if (n < QSV_N_MIN || n > QSV_N_MAX)
         return fail(QSV_ERR_INVALID_ARG, "n out of [10, 34] for the fixed-scratch reduction");
     size_t need = 0;
-    cudaError_t e = qsv::launch_reduce_noalloc(state, n, dtype, out_dev, sm_count(), (cudaStream_t)stream, &need);
+    cudaError_t e = qsv::launch_reduce_noalloc(state, n, dtype, out_dev, (cudaStream_t)stream, &need);
     if (need > qsv::noalloc_reduce_capacity())
         return fail(QSV_ERR_SCRATCH, "state needs " + std::to_string(need) + " B of block partials, fixed scratch holds " +
                                          std::to_string(qsv::noalloc_reduce_capacity()) + " B");
