@@ -331,10 +331,15 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---------------------------------------------------------------- chunk probabilities
-// One warp per chunk of 2^cb amplitudes (cb >= CHUNK_WARP_MIN): 16-byte loads, eight in flight per lane, no block
-// barriers. Grid-strided over the chunks.
+// What bounds it: the read of the state. Small chunks (256 amplitudes to 8 KiB) take a warp each, grid-strided; larger
+// ones a block each, which the hardware deals out as blocks finish. A warp per chunk had been used up to 2^13 amplitudes,
+// where the last turn of the grid-stride is a good part of the time and a few chunks leave the SMs idle. Device time,
+// warp / block: chunks of 2^12 complex64 amplitudes (the default) 8.6 / 5.0 us at 18 qubits, 24.5 / 23.2 at 24, 322 / 290
+// at 28; 2^11: 26.7 / 23.2 at 24; 2^10: 24.8 / 29.9; of 2^12 complex128 amplitudes 48.6 / 43.7 us at 24 qubits, 622 / 582
+// at 28, 2^10: 43.8 / 41.6 at 24, 2^9: 43.9 / 62.0.
 #define CHUNK_WARP_MIN 8           // 256 complex64 amplitudes: 4 loads per lane
-#define CHUNK_WARP_MAX 13
+#define CHUNK_WARP_BYTES 8192
+// One warp per chunk of 2^cb amplitudes: 16-byte loads, eight in flight per lane, no block barriers.
 __device__ __forceinline__ double prob16(const float4 &v) { return prob(v.x, v.y) + prob(v.z, v.w); }
 __device__ __forceinline__ double prob16(const double2 &v) { return v.x * v.x + v.y * v.y; }
 template <class A, bool AL>
@@ -360,18 +365,25 @@ __global__ void __launch_bounds__(RED_THREADS)
     }
 }
 
-// one block per chunk (any other chunk size)
+// One block per chunk (any other chunk size), eight loads in flight per thread. (One at a time with 64-bit indices, a
+// whole 24-qubit complex128 state in one chunk took 12.3 ms, with 32-bit ones 9.3.)
 template <class A>
 __global__ void __launch_bounds__(RED_THREADS)
     chunk_probs_kernel(const A *__restrict__ state, int cb, double *__restrict__ out) {
     __shared__ double s[RED_THREADS];
-    const int64_t base = (int64_t)blockIdx.x << cb;
+    const A *p = state + ((int64_t)blockIdx.x << cb);
     const int64_t len = 1ll << cb;
     double acc = 0.0;
-    for (int64_t i = threadIdx.x; i < len; i += RED_THREADS) {
-        const A a = state[base + i];
-        acc += (double)a.x * a.x + (double)a.y * a.y;
+    auto add = [&](const A &a) { acc += (double)a.x * a.x + (double)a.y * a.y; };
+    int64_t i = threadIdx.x;
+    for (; i + 7 * RED_THREADS < len; i += 8 * RED_THREADS) {
+        A a[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) a[k] = p[i + k * RED_THREADS];
+#pragma unroll
+        for (int k = 0; k < 8; k++) add(a[k]);
     }
+    for (; i < len; i += RED_THREADS) add(p[i]);
     s[threadIdx.x] = acc;
     __syncthreads();
     for (int w = RED_THREADS / 2; w > 0; w >>= 1) {
@@ -388,7 +400,7 @@ __global__ void __launch_bounds__(RED_THREADS)
 // amplitude, each the first whose running FP64 sum exceeds what is left of the draw.
 // What bounds it: the read of the state for the chunk probabilities. A scan of 2^16 values in one block and one
 // thread per shot adding up to 4096 amplitudes one after the other took 1.20 ms for 1024 shots of 28 qubits
-// (HBM floor 0.33 ms); now 0.36 ms, and 38 instead of 440-530 us at 12-20 qubits.
+// (HBM floor 0.33 ms); now 0.33 ms, and 38 instead of 440-530 us at 12-20 qubits.
 #define SCAN_BITS 12
 #define SCAN_THREADS 1024
 __device__ __forceinline__ double warp_scan(double v, int lane) {       // inclusive
@@ -691,7 +703,7 @@ cudaError_t launch_reduce_noalloc(const void *state, int n, int dtype, double *o
 template <class A>
 static cudaError_t launch_chunk_probs_t(const A *state, int n, int cb, double *out, int nsm, cudaStream_t stream) {
     const int64_t nc = 1ll << (n - cb);
-    if (cb >= CHUNK_WARP_MIN && cb <= CHUNK_WARP_MAX) {
+    if (cb >= CHUNK_WARP_MIN && sizeof(A) << cb <= CHUNK_WARP_BYTES) {
         int64_t grid = (nc + RED_THREADS / 32 - 1) / (RED_THREADS / 32);
         if (grid > (int64_t)nsm * 8) grid = (int64_t)nsm * 8;
         if (aligned16(state))
