@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(RED_THREADS)
 // amplitude, each the first whose running FP64 sum exceeds what is left of the draw.
 // What bounds it: the read of the state for the chunk probabilities. A scan of 2^16 values in one block and one
 // thread per shot adding up to 4096 amplitudes one after the other took 1.20 ms for 1024 shots of 28 qubits
-// (HBM floor 0.33 ms); now 0.33 ms, and 38 instead of 440-530 us at 12-20 qubits.
+// (HBM floor 0.33 ms); now 0.34 ms, and 38 instead of 440-530 us at 12-20 qubits.
 #define SCAN_BITS 12
 #define SCAN_THREADS 1024
 __device__ __forceinline__ double warp_scan(double v, int lane) {       // inclusive

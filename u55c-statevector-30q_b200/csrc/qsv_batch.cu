@@ -5,7 +5,7 @@
 // every segment, in order) runs inside one CTA's shared memory: one HBM read and one HBM write per
 // circuit instead of one per pass. The kernel is the sweep kernel's pipeline with circuits in place of
 // tiles: a producer warp streams circuit states in and out with bulk-async copies (three in flight), the
-// consumer warps run each circuit's phases with the shared op code (qsv_ops.cuh). The per-circuit programs
+// consumer warps run each circuit's phases with the interpreter's code (qsv_interp.cuh). The per-circuit programs
 // (phases and ops) live in a caller-provided device workspace, uploaded once and replayable (the launch is
 // capturable in a CUDA graph).
 #include <cuda_runtime.h>

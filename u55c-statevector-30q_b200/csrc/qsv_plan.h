@@ -23,8 +23,8 @@
 //   lane_bits[0..1]     -> lane bits 3, 4
 //   reg_bits[0..RB-1]   -> register index bits (2^RB float4 per thread)
 //   warp_bits[..]       -> warp index bits
-// An op can run in a phase when its target is tile bit 0..3, a register bit or a lane bit of that phase;
-// controls may sit anywhere in the window.
+// An op can run in a phase when its target is tile bit 0..3, a register bit or a lane bit of that phase, or, on
+// the interpreters, when it is diagonal; controls may sit anywhere in the window.
 #pragma once
 #ifdef __CUDACC_RTC__
 // compiled at run time by NVRTC (sweep kernels specialised to one structure): no host headers there
@@ -87,7 +87,7 @@ typedef unsigned long long uint64_t;
 #define QSV_SLOT_COMP 0         // tile bit 0 (inside a float4)
 #define QSV_SLOT_REG0 1         // 1 + r: register bit r
 #define QSV_SLOT_LANE0 8        // 8 + l: lane bit l (warp shuffle)
-#define QSV_SLOT_BASE 7         // streaming interpreter: diagonal op on a tile bit of the item base
+#define QSV_SLOT_BASE 7         // interpreters: diagonal op on a warp bit; streaming form: on a bit of the item base
 
 // 96 bytes, 16-byte aligned: the matrices are four 16-byte vectors and every field a kernel reads is in
 // the 16 bytes at offset 64 (one vector load per op in the streaming interpreter).

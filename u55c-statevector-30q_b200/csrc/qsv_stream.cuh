@@ -5,8 +5,9 @@
 // of it: a thread takes items of 8 float4 = 16 amplitudes on tile bits {0, q[0], q[1], q[2]} (float4 r holds
 // item base | r.0 * 2^q[0] | r.1 * 2^q[1] | r.2 * 2^q[2]), applies the group's ops to them in registers and
 // stores them back. Any target bit can be an item bit, so a sweep needs no phase layouts, and ops on tile
-// bit 0 and diagonal ops on any bit ride along with the group. The ops run through the phase interpreter's
-// code paths (reg_op with the item bits as register bits 0-2, comp_op_fast), so every value is the same.
+// bit 0 and diagonal ops on any bit ride along with the group. The ops run through code paths of their own
+// (reg_op with the item bits as register bits 0-2, comp_op_fast in qsv_ops.cuh) with the same multiply-add
+// chain as the phase interpreter's, so every value is the same.
 //
 // Two ways to run a group's ops on an item: stream_op reads each op's slot and variant at run time (one
 // dispatch per op and item); stream_op_fixed takes them as template arguments (straight-line code for a

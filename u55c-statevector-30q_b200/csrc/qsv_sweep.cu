@@ -33,8 +33,8 @@ namespace dev {
 // Device status word: kernels OR a bit in when a bounded wait gives up (1 = mbarrier wait timeout).
 __device__ int g_status = 0;
 
-// The interpreter: the sweep's phases and ops are read at run time (op table in shared memory), one code
-// path per op variant selected by a switch.
+// The interpreter: the sweep's phases and ops are read at run time (op table in shared memory, expanded once per
+// launch), each op's code path found by a short chain of branches (qsv_interp.cuh).
 struct InterpBody {
     using Amp = float2;
     static constexpr int kHalfBits = 1;
@@ -88,10 +88,11 @@ struct InterpBody {
 // The tile stays in shared memory and each group of ops (plan_stream) is one round trip of it: a thread
 // takes items of 8 float4 = 16 amplitudes on tile bits {0, q[0], q[1], q[2]} (float4 r holds item base |
 // r.0 * 2^q[0] | r.1 * 2^q[1] | r.2 * 2^q[2]), applies the group's ops to them in registers and stores them
-// back. Only one item's 32 floats are live across the run-time dispatch of an op (the phase interpreter
-// keeps 64), any target bit can be an item bit, so a sweep needs no phase layouts, and ops on tile bit 0
-// and diagonal ops on any bit ride along with the group. The ops run through the phase interpreter's code
-// paths (reg_op with the item bits as register bits 0-2, comp_op_fast), so every value is the same.
+// back. One item's 32 floats are live across the run-time dispatch of an op (as many as a thread of the phase
+// interpreter keeps), any target bit can be an item bit, so a sweep needs no phase layouts, and ops on tile
+// bit 0 and diagonal ops on any bit ride along with the group. The ops run through code paths of their own
+// (reg_op with the item bits as register bits 0-2, comp_op_fast in qsv_ops.cuh) with the same multiply-add
+// chain as the phase interpreter's, so every value is the same.
 
 static_assert(sizeof(QsvOp) == 96 && offsetof(QsvOp, cm_thr) == 64 && offsetof(QsvOp, cm_reg) == 68 &&
                   offsetof(QsvOp, cls0) == 72 && offsetof(QsvOp, variant) == 76 && offsetof(QsvOp, m1) == 32,

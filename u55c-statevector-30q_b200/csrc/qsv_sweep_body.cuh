@@ -14,7 +14,7 @@
 //     a tile: a thread runs a phase of the other tile while the slowest threads finish their stores, so the
 //     phase round trips of one tile overlap the arithmetic of the other without a second register set.
 // Body is the interpreter (qsv_sweep.cu: op table read at run time) or a kernel specialised to one sweep
-// structure (qsv_jit.cpp: ops fixed at compile time). Both run the same arithmetic (qsv_ops.cuh).
+// structure (qsv_jit.cpp: ops fixed at compile time). Both run the same arithmetic (qsv_packed.cuh).
 // The tile addressing is the reference's (host/sv/model.py:25-40, sv_engine.cpp:61-84,116): tile T's
 // base is pdep(T, free bits) and sub-block s sits at base | pdep(s, H).
 #pragma once

@@ -4,14 +4,14 @@
 // precision study (a 32-qubit complex128 state is 64 GiB). Same sweep plans, addressing and staging
 // pipeline as the complex64 engine (qsv_sweep_body.cuh), with one 16-byte amplitude per thread slot: tile
 // bits 0-2 are lane bits 0-2 (with the swizzled layout any of bits 0-5 can be register bits), two chosen
-// tile bits are lane bits 3-4, four are register bits and the rest warp bits (windows of at most 12 qubits:
-// 3 x 64 KiB buffers).
+// tile bits are lane bits 3-4, three are register bits (8 amplitudes per thread) and the other kw - 8 are warp
+// bits (windows of at most 12 qubits: 3 x 64 KiB buffers).
 // What bounds it: staging first. A window of short runs staged with one bulk copy per run (256 copies of
 // 256 bytes per 64 KiB tile each way) moved 0.9 TB/s whatever its ops; with one tensor-map box per tile the
 // same sweeps are bound by their ops. Those run in one tight loop per op variant and slot over all of a
 // thread's pairs, coefficients in registers (a class test per pair cost as much as the arithmetic).
 // A 27-qubit random-layer circuit with Toffolis, depth 8 (41 sweeps, HBM floor 27 ms): 189 ms before, 107 ms
-// with the loops, 53 ms with the tensor maps and swizzled layouts as well.
+// with the loops, 53 ms with the tensor maps and swizzled layouts as well, 41 ms with expanded records and 16 warps.
 // Every pair update is the canonical fused-multiply-add chain in double precision
 //   y0.re = fma(m00.re, x0.re, fma(-m00.im, x0.im, fma(m01.re, x1.re, -(m01.im * x1.im))))  (etc.)
 // which the CPU oracle's complex128 engine writes identically, so results agree value for value; the
